@@ -1,0 +1,85 @@
+"""The block-bitmap counting path (tc_bits.cu) at the sizes where it can go wrong, against the
+oracle's forward-intersection counter: rows at the table bound and at the bounds of the row
+conversion's kernels, bitmaps narrower and wider than the graph, tail ids over several passes."""
+import numpy as np
+import pytest
+
+import trust_gb300 as T
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _csr(rows, n):
+    beg = np.zeros(n + 1, dtype=np.int64)
+    for v, r in rows.items():
+        beg[v + 1] = len(r)
+    beg = np.cumsum(beg)
+    adj = np.zeros(int(beg[-1]), dtype=np.int32)
+    for v, r in rows.items():
+        adj[beg[v]:beg[v + 1]] = r
+    return beg, adj
+
+
+def _check(beg, adj, lo=None, hi=None):
+    db, da = torch.from_numpy(beg).cuda(), torch.from_numpy(adj).cuda()
+    expect = O.count_forward_sorted_range(beg, adj, 0, beg.size - 1, 2, 8)
+    d = np.diff(beg)
+    src = np.repeat(np.arange(d.size), d)
+    sel = d[src] >= 2
+    with T.Context() as ctx:
+        for _ in range(2):
+            r = T.count_csr(db, da, ctx=ctx, direction_split=1)
+            assert r.triangles == expect and r.direction_split == 1
+            assert r.wedges == int(np.minimum(d[adj], d[src])[sel].sum())
+        n = beg.size - 1
+        cut = [0, n // 3, n // 2 + 1, n]
+        parts = [T.count_csr(db, da, ctx=ctx, direction_split=1, row_range=(a, b)).triangles
+                 for a, b in zip(cut[:-1], cut[1:])]
+        assert sum(parts) == expect
+        assert T.count_csr(db, da, ctx=ctx, direction_split=1, schedule=T.SCHED_TUNED).triangles == expect
+        assert T.count_csr(db, da, ctx=ctx, schedule=T.SCHED_PLAIN).triangles == expect
+
+
+@pytest.mark.parametrize("n", [129, 130, 131, 200, 513, 514, 700, 1100])
+def test_complete_graphs(n):
+    """Row v = v+1..n-1: rows of every length up to n-1 (128 / 129: the table bound; 32 / 33 and
+    512 / 513: the conversion kernels' bounds)."""
+    rows = {v: np.arange(v + 1, n) for v in range(n)}
+    _check(*_csr(rows, n))
+
+
+@pytest.mark.parametrize("scale,ef,a", [(10, 64, 0.57), (13, 48, 0.45), (15, 24, 0.7), (17, 16, 0.57)])
+def test_rmat(scale, ef, a):
+    b = (0.95 - a) / 2
+    beg, adj = T.build_csr(T.gen_rmat(scale, ef, a, b, b, seed=scale), 1 << scale)
+    _check(beg.cpu().numpy(), adj.cpu().numpy())
+
+
+@pytest.mark.parametrize("n,hubs,row", [(300_000, 40, 300), (600_000, 30, 1500), (500_000, 12, 3000),
+                                        (400_000, 3, 8192)])
+def test_tails(n, hubs, row):
+    """Rows whose columns mostly lie beyond the bitmap (one reader each): tails of one and of several
+    passes; the hubs also point at each other and share some columns."""
+    rng = np.random.default_rng(n + hubs)
+    rows = {}
+    shared = rng.choice(np.arange(hubs, n), size=row // 4, replace=False)
+    for h in range(hubs):
+        mine = rng.choice(np.arange(hubs, n), size=row - shared.size - (hubs - 1 - h), replace=False)
+        rows[h] = np.unique(np.concatenate([np.arange(h + 1, hubs), shared, mine]))[:row]
+    for v in range(hubs, n, 7):  # many short rows: popular columns and a few of their own
+        rows[v] = np.unique(rng.integers(hubs, n, size=rng.integers(1, 5)))
+    beg, adj = _csr(rows, n)
+    _check(beg, adj)
+
+
+@pytest.mark.parametrize("row", [8192, 8193])
+def test_longest_row(row):
+    """One row of 8192 entries (the longest the conversion groups) and of 8193 (the hash tables)."""
+    n = 20_000
+    rng = np.random.default_rng(row)
+    rows = {0: np.sort(rng.choice(np.arange(1, n), size=row, replace=False))}
+    for v in range(1, 3000):
+        rows[v] = np.unique(rng.integers(v + 1, n, size=rng.integers(1, 300)))
+    _check(*_csr(rows, n))

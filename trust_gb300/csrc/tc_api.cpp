@@ -18,6 +18,7 @@
 #include <string>
 #include <vector>
 
+#include "tc_bits.h"
 #include "tc_count.h"
 #include "tc_internal.h"
 #include "tc_model.h"
@@ -104,6 +105,10 @@ void ctx_release(trust_tc_ctx *c) {
   cudaFree(c->d_split_cbeg);
   cudaFree(c->d_split_rowmap);
   cudaFree(c->d_split_adj);
+  cudaFree(c->d_bits_cols);
+  cudaFree(c->d_bits_ent);
+  cudaFree(c->d_bits_desc);
+  cudaFree(c->d_bits_units);
   cudaFree(c->d_beg);
   cudaFree(c->d_adj);
   for (auto &ev : c->ev)
@@ -305,6 +310,13 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
       same && g.min_deg == 2 && g.rows > 0 &&
       (o.direction_split == 1 || (learned && h.max_out_degree >= 64 && g.mA >= TC_LEARNED_MIN_ARCS &&
                                   (!fused || (double)h.long_arcs >= TC_LEARNED_MIN_LONG_FRAC * (double)g.mA)));
+  // with the split, rows longer than BITS_TABLE_MIN are counted as block bitmaps (tc_bits.cu) unless
+  // the caller asks for something of the hash tables' own: cycles, hub clusters, CTA bounds below
+  const bool bits_ok = consider && !o.record_cycles && o.hub_cluster == 0 && !o.test_wait_expiry &&
+                       cfg.cta_max >= BITS_TABLE_MIN && bits_eligible(g, h.max_out_degree);
+  unsigned long long plan_wedges = 0;
+  BitsPlan bits;
+  bool use_bits = false;
   if (consider) {
     const float *d_model = nullptr;
     if (learned) {
@@ -314,7 +326,7 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     // (the pass also checks that rows are duplicate-free, which the split needs); with a model,
     // the class histogram under its decisions follows on the stream before the one readback
     rc = split_plan(c, g.begA, g.adjA, g.rows, g.mA, st, d_model, cfg.warp_max, cfg.cta_max, TC_PROMOTE_LOG2,
-                    cfg.threads / 32, ctl, row_lo, row_hi);
+                    cfg.threads / 32, ctl, row_lo, row_hi, bits_ok ? BITS_TABLE_MIN : 0);
     if (rc) return rc;
     if (d_model) {
       dec = c->d_dec;
@@ -346,6 +358,14 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
       split = sorted && saved_ms > 1.5 * cost_ms;
     } else {
       split = sorted && split_pays(plan.w_all, plan.w_min, g.mA, g.rows);
+    }
+    if (split && bits_ok) {
+      plan_wedges = plan.w_min;
+      rc = bits_prepare(c, g.begA, g.adjA, g.rows, g.mA, row_lo, row_hi < 0 ? g.rows : row_hi, plan, h.max_out_degree,
+                        st, &bits);
+      if (rc == TRUST_TC_E_NOMEM) split = 0;  // no room for the blocks (allocated first): count unsplit
+      else if (rc) return rc;
+      use_bits = rc == TRUST_TC_OK;
     }
   }
   // a tile job (three CSRs, duplicate-free tables and probe rows): the same split, decided by the
@@ -382,7 +402,7 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
   // one CTA 3.44 s, clusters of 2 / 4 CTAs 4.30 / 5.77 s, global tables 3.63 s.
   int hub_log2C = -1, hub_max_log2 = 0, hub_clusters = 0;
   const int64_t table_max = g.max_deg_A > 0 ? g.max_deg_A : h.max_out_degree;  // largest table row
-  if (h.class_count[TC_CLASS_HUGE] > 0 && o.hub_cluster >= 0) {
+  if (h.class_count[TC_CLASS_HUGE] > 0 && o.hub_cluster >= 0 && !use_bits) {
     const int tlog2 = std::max(ceil_log2_size(2 * table_max), 6);
     if (o.hub_cluster > 0) {
       hub_log2C = ceil_log2_size(o.hub_cluster);
@@ -397,7 +417,7 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     a.hub_max_degree = 1 << (hub_max_log2 - 1);
     hub_clusters = std::max(1, std::min(h.class_count[TC_CLASS_HUGE], (2 * c->num_sms) >> hub_log2C));
   }
-  if (h.class_count[TC_CLASS_HUGE] > 0 && table_max > a.hub_max_degree) {
+  if (h.class_count[TC_CLASS_HUGE] > 0 && table_max > a.hub_max_degree && !use_bits) {
     a.huge_log2 = ceil_log2_size(2 * table_max);
     size_t per = (size_t)4 << a.huge_log2;
     size_t budget = (size_t)1 << 31;  // 2 GiB of spill tables at most
@@ -410,14 +430,16 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
   // shared memory sized to what this graph needs: warp tables, plus a CTA table only as large as
   // the largest CTA-class row present; the rest of the SM's unified memory stays L1
   // warp tables sized to the largest row a warp can get here (>= 128 slots: 4G for G32 groups)
-  const int warp_slots = 1 << std::max(ceil_log2_size(2 * std::min<int64_t>(table_max, cfg.warp_max)), 7);
+  // (with block bitmaps, only rows of up to BITS_TABLE_MIN entries are left to these tables)
+  const int64_t longest = use_bits ? std::min<int64_t>(table_max, BITS_TABLE_MIN) : table_max;
+  const int warp_slots = 1 << std::max(ceil_log2_size(2 * std::min<int64_t>(longest, cfg.warp_max)), 7);
   size_t smem = (size_t)4 * warp_slots * (cfg.threads / 32);
   // quotient tables for the CTA class when every key and probe id has at most 26 bits; the CTA
   // table's bytes then also hold a 512-byte overflow list (tc_count.cu, TC_Q16_OVERFLOW)
   const int key_bits = ceil_log2_size(std::max<int64_t>(std::max(g.boundA, g.boundC), 2));
   const bool q16 = key_bits <= 26;
   if (h.class_count[TC_CLASS_CTA] > 0) {
-    const int64_t dcta = std::min<int64_t>(h.max_out_degree, cfg.cta_max);
+    const int64_t dcta = std::min<int64_t>(use_bits ? longest : h.max_out_degree, cfg.cta_max);
     smem = std::max(smem, ((size_t)4 << std::max(ceil_log2_size(2 * dcta), 6)) + (q16 ? 512 : 0));
   }
   int blocks = cfg.blocks;
@@ -454,6 +476,7 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
   a.test_wait_expiry = o.test_wait_expiry;
   a.key_bits = q16 ? key_bits : 0;
   a.cta_table_bytes = (int)smem;
+  a.table_min = use_bits ? BITS_TABLE_MIN : 0;
   if (h.class_count[TC_CLASS_CTA] > 0) {
     // long-row lists: one per CTA, as long as the largest CTA-class row
     const int cap = (int)std::min<int64_t>(h.max_out_degree, cfg.cta_max);
@@ -470,6 +493,10 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     rc = launch_hub(same, a, hub_max_log2, hub_log2C, hub_clusters, st);
     if (rc) return rc;
   }
+  if (use_bits) {
+    rc = bits_launch(c, bits, g.adjA, ctl, st);
+    if (rc) return rc;
+  }
   rc = launch_count(same, a, blocks, cfg.threads, smem, st);
   if (rc) return rc;
   TC_CUDA_TRY(cudaEventRecord(c->ev[3], st));
@@ -478,7 +505,8 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
   memset(&rb, 0, sizeof rb);
   float t_build = 0;
   int rb_status = 0;  // TC_DEV_* bits of the second pass
-  if (split) {
+  const bool second_pass = split && !use_bits;
+  if (second_pass) {
     // Second pass: arcs (v,u) with d(u) > d(v), hashed on u's row, streaming the sources' rows (a
     // tile job: tables from C's rows, probe rows from A's).  It runs on the context's second stream
     // with a second context's scratch while the first pass still counts: the scheduling pass's
@@ -503,7 +531,7 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
   TC_CUDA_TRY(cudaEventElapsedTime(&t_kernel, c->ev[1], c->ev[3]));
   TC_CUDA_TRY(cudaEventElapsedTime(&t_count, c->ev[2], c->ev[3]));
   TC_CUDA_TRY(cudaEventElapsedTime(&t_call, c->ev[0], c->ev[4]));
-  if (split) {  // classification (counting) to the end of whichever pass ends last
+  if (second_pass) {  // classification (counting) to the end of whichever pass ends last
     float t_end_b = 0, t_count_b = 0;
     TC_CUDA_TRY(cudaEventElapsedTime(&t_end_b, c->ev[1], c->ev_split[2]));
     TC_CUDA_TRY(cudaEventElapsedTime(&t_count_b, c->ev[2], c->ev_split[2]));
@@ -511,7 +539,7 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     t_count = std::max(t_count, t_count_b);
   }
   r->triangles = done.count + rb.triangles;
-  r->wedges = (int64_t)done.wedges + rb.wedges;
+  r->wedges = use_bits ? (int64_t)plan_wedges : (int64_t)done.wedges + rb.wedges;
   r->kernel_seconds = t_kernel * 1e-3;
   // the counting kernels' wall span: from the first pass's first counting launch to the end of
   // whichever pass ends last (the two passes run at the same time on two streams)

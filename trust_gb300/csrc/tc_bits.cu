@@ -1,0 +1,723 @@
+// tc_bits.cu — block-bitmap rows: the direction split's counting path on skewed graphs.
+//
+// After the direction split an arc (v,u) is counted by streaming the shorter of its two rows
+// against a table of the longer one.  On skewed graphs nearly all of that work lies in rows whose
+// entries are a small set of popular columns, so this path renumbers the columns by popularity
+// (in-degree) and stores every row as 16-column blocks: one 32-bit entry (block << 17 | bit mask)
+// per block present, popular blocks first.  The table of a row is then a plain bitmap in shared
+// memory, indexed by block: a lookup is one 16-bit load with no hashing, no key compare and no
+// collision, and one AND + popcount settles up to 16 probes.  R-MAT 20 ef16: 0.46 entries per
+// probe (a = 0.57), 0.26 (a = 0.70).  Columns beyond the bitmap ("tail" entries, the unpopular
+// ones) stay plain ids after the row's blocks and are looked up in a small hash set.
+//
+// The rows must be duplicate-free (the split already requires it), so |N+(v) ∩ N+(u)| is the same
+// number from either side and in any column numbering.
+#include <algorithm>
+
+#include "tc_bits.h"
+#include "tc_count.h"
+#include "tc_internal.h"
+
+namespace tc {
+
+namespace {
+
+typedef unsigned int u32;
+
+// ---- column popularity -----------------------------------------------------------------------
+__global__ void indeg_kernel(const int32_t *__restrict__ adj, int64_t m, u32 *__restrict__ indeg) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += 4 * stride) {
+    int u[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) u[r] = i + r * stride < m ? tc_ld_nc(adj + i + r * stride) : -1;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (u[r] >= 0) atomicAdd(indeg + u[r], 1u);
+  }
+}
+
+// Popularity bucket, most popular first: 8 buckets per doubling of the in-degree.
+__device__ __forceinline__ int pop_bucket(u32 x) {
+  if (x == 0) return 255;
+  const int e = 31 - __clz(x);
+  const int mant = e >= 3 ? (int)(x >> (e - 3)) & 7 : (int)(x << (3 - e)) & 7;
+  return 254 - min(254, e * 8 + mant);
+}
+
+constexpr int RK_TILE = 4096;
+
+__global__ void __launch_bounds__(256) rank_hist_kernel(const u32 *__restrict__ indeg, int64_t n, u32 *__restrict__ counts,
+                                                        u32 ntiles) {
+  __shared__ u32 h[256];
+  h[threadIdx.x] = 0;
+  __syncthreads();
+  const int64_t base = (int64_t)blockIdx.x * RK_TILE;
+  for (int r = 0; r < RK_TILE / 256; ++r) {
+    const int64_t i = base + r * 256 + threadIdx.x;
+    const int b = i < n ? pop_bucket(indeg[i]) : 256;
+    const unsigned peers = __match_any_sync(TC_FULL_MASK, b);
+    if (b < 256 && (peers & tc_lanemask_lt()) == 0) atomicAdd(&h[b], (u32)__popc(peers));
+  }
+  __syncthreads();
+  counts[(size_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
+}
+
+// rank[w] = position of column w, popular buckets first (any order inside a bucket and tile).
+__global__ void __launch_bounds__(256) rank_scatter_kernel(const u32 *__restrict__ indeg, int64_t n,
+                                                           const u32 *__restrict__ offs, u32 ntiles,
+                                                           u32 *__restrict__ rank) {
+  __shared__ u32 cur[256];
+  cur[threadIdx.x] = offs[(size_t)threadIdx.x * ntiles + blockIdx.x];
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int64_t base = (int64_t)blockIdx.x * RK_TILE;
+  for (int r = 0; r < RK_TILE / 256; ++r) {
+    const int64_t i = base + r * 256 + threadIdx.x;
+    const int b = i < n ? pop_bucket(indeg[i]) : 256;
+    const unsigned peers = __match_any_sync(TC_FULL_MASK, b);
+    const int leader = __ffs(peers) - 1;
+    u32 at = 0;
+    if (b < 256 && lane == leader) at = atomicAdd(&cur[b], (u32)__popc(peers));
+    at = __shfl_sync(TC_FULL_MASK, at, leader);
+    if (b < 256) rank[i] = at + __popc(peers & tc_lanemask_lt());
+  }
+}
+
+// ---- rows to blocks --------------------------------------------------------------------------
+// Row v owns entries from row_start(v): 16-byte aligned, room for its d entries and the zero
+// entries that pad its blocks to a multiple of four (m + 6 n entries in all).
+__host__ __device__ __forceinline__ u32 row_start(int64_t beg, int64_t v) { return (u32)((beg + 6 * v + 3) & ~3ll); }
+
+// Position (0..31) of the n-th (0-based) set bit of mask; mask must have more than n set bits.
+__device__ __forceinline__ int nth_bit(unsigned mask, int n) {
+  int pos = 0;
+#pragma unroll
+  for (int step = 16; step >= 1; step >>= 1) {
+    const int cnt = __popc(mask & ((1u << step) - 1u));
+    if (n >= cnt) {
+      n -= cnt;
+      mask >>= step;
+      pos += step;
+    }
+  }
+  return pos;
+}
+
+// Place of a row's e-th block (of nd4 * 4, padding included).  Blocks are laid out in chunks of 32,
+// transposed: eight lanes read a chunk with one 16-byte load each, and the c-th 16-bit lookups of
+// the eight then go to consecutive blocks, whose words share few banks where a row is dense.
+__device__ __forceinline__ int entry_place(int e, int nd4) {
+  const int lanes = min(8, nd4 - (e >> 5 << 3)), r = e & 31;
+  return (e & ~31) + (lanes == 8 ? (r & 7) * 4 + (r >> 3) : (r % lanes) * 4 + r / lanes);
+}
+
+constexpr int BITS_WARP_ROW = 512;  // rows up to this are converted by a warp, above by a CTA
+
+// Rows of at most 32 entries: a warp takes 32 consecutive rows, packs as many whole rows as fit
+// its lanes, and groups the lanes of a row that fall into one block with a match.  Longer rows are
+// listed (longs: warp rows from the front, CTA rows from the back).
+__global__ void __launch_bounds__(256) bits_short_kernel(const int64_t *__restrict__ beg, const int32_t *__restrict__ adj,
+                                                         int64_t n, const u32 *__restrict__ rank, int nb,
+                                                         u32 *__restrict__ ent, int4 *__restrict__ desc,
+                                                         int *__restrict__ longs, u32 *__restrict__ nlongs) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = tc_lanemask_lt();
+  const unsigned upto = 0xffffffffu >> (31 - lane);
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t v0 = warp * 32; v0 < n; v0 += nwarps * 32) {
+    const int64_t v = v0 + lane;
+    int b = 0, d = 0;
+    if (v < n) {
+      const long long lo = tc_ld_nc(beg + v);
+      b = (int)lo;
+      d = (int)(tc_ld_nc(beg + v + 1) - lo);
+      if (d == 0) desc[v] = make_int4(0, 0, 0, 0);
+    }
+    const unsigned w1 = __ballot_sync(TC_FULL_MASK, d > 32 && d <= BITS_WARP_ROW);
+    const unsigned w2 = __ballot_sync(TC_FULL_MASK, d > BITS_WARP_ROW);
+    if (w1 | w2) {
+      u32 at1 = 0, at2 = 0;
+      if (lane == 0) {
+        if (w1) at1 = atomicAdd(nlongs, (u32)__popc(w1));
+        if (w2) at2 = atomicAdd(nlongs + 1, (u32)__popc(w2));
+      }
+      at1 = __shfl_sync(TC_FULL_MASK, at1, 0);
+      at2 = __shfl_sync(TC_FULL_MASK, at2, 0);
+      if (w1 >> lane & 1) longs[at1 + __popc(w1 & lt)] = (int)v;
+      if (w2 >> lane & 1) longs[n - 1 - (int64_t)(at2 + __popc(w2 & lt))] = (int)v;
+    }
+    const int sd = d <= 32 ? d : 0;
+    int incl = sd;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(TC_FULL_MASK, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const int excl = incl - sd;
+    const int tot = __shfl_sync(TC_FULL_MASK, incl, 31);
+    for (int base = 0; base < tot;) {
+      const bool in = sd > 0 && excl >= base && incl <= base + 32;
+      const unsigned inm = __ballot_sync(TC_FULL_MASK, in);
+      const unsigned starts = __reduce_or_sync(TC_FULL_MASK, in ? 1u << (excl - base) : 0u);
+      const int wend = __reduce_max_sync(TC_FULL_MASK, in ? incl : 0);
+      const bool valid = lane < wend - base;
+      const int own = valid ? nth_bit(inm, __popc(starts & upto) - 1) : 0;
+      const int bj = __shfl_sync(TC_FULL_MASK, b, own);
+      const int ex = __shfl_sync(TC_FULL_MASK, excl, own) - base;
+      const int dj = __shfl_sync(TC_FULL_MASK, sd, own);
+      const u32 w = valid ? rank[tc_ld_nc(adj + bj + (lane - ex))] : 0u;
+      const u32 blk = w >> 4;
+      const bool direct = valid && blk < (u32)nb, tail = valid && !direct;
+      const u32 key = direct ? ((u32)own << 16 | blk) : 0x80000000u | (u32)lane;
+      const unsigned peers = __match_any_sync(TC_FULL_MASK, key);
+      const u32 mask = __reduce_or_sync(peers, 1u << (w & 15u));
+      const unsigned lead = __ballot_sync(TC_FULL_MASK, direct && (peers & lt) == 0);
+      const unsigned tails = __ballot_sync(TC_FULL_MASK, tail);
+      if (valid) {
+        const unsigned mine = (dj == 32 ? 0xffffffffu : ((1u << dj) - 1u)) << ex;
+        const int nd = __popc(lead & mine), pad = (nd + 3) & ~3;
+        const u32 s = row_start(bj, v0 + own);
+        if (lead >> lane & 1) ent[s + entry_place(__popc(lead & mine & lt), pad >> 2)] = blk << 17 | mask;
+        if (tail) ent[s + pad + __popc(tails & mine & lt)] = w;
+        if (lane == ex) {
+          for (int k = nd; k < pad; ++k) ent[s + entry_place(k, pad >> 2)] = 0;
+          desc[v0 + own] = make_int4((int)s, pad, __popc(tails & mine), dj);
+        }
+      }
+      base = wend;
+    }
+  }
+}
+
+// Grouping table of a long row: slots (block << 17 | mask), 0 = empty; T = a power of two >= 2 d.
+// The lower half is indexed by the block itself (popular blocks come out in order, so that a warp
+// reading the row later touches neighbouring words of a table), the upper half by a hash of the
+// other blocks; a row has at most T/2 blocks, so the upper half never overflows.
+__device__ __forceinline__ void group_insert(u32 *tab, int T, u32 w) {
+  const u32 blk = w >> 4, bit = 1u << (w & 15u), e = blk << 17;
+  const u32 half = (u32)T >> 1;
+  u32 h = blk < half ? blk : half + ((blk * 0x9E3779B1u >> 12) & (half - 1));
+  for (int it = 0; it < T; ++it) {
+    const u32 prev = atomicCAS(tab + h, 0u, e | bit);
+    if (prev == 0u) return;
+    if ((prev ^ e) < 0x10000u) {
+      atomicOr(tab + h, bit);
+      return;
+    }
+    h = half + ((h + 1) & (half - 1));
+  }
+}
+
+__device__ __forceinline__ int group_slots(int d) {
+  int T = 64;
+  while (T < 2 * d) T <<= 1;
+  return T;
+}
+
+// A warp per row of 33..BITS_WARP_ROW entries.
+__global__ void __launch_bounds__(256) bits_warp_kernel(const int64_t *__restrict__ beg, const int32_t *__restrict__ adj,
+                                                        const u32 *__restrict__ rank, int nb, u32 *__restrict__ ent,
+                                                        int4 *__restrict__ desc, const int *__restrict__ longs,
+                                                        const u32 *__restrict__ nlongs) {
+  __shared__ u32 tabs[8][2 * BITS_WARP_ROW];
+  u32 *tab = tabs[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = tc_lanemask_lt();
+  const u32 nl = nlongs[0];
+  const u32 nwarps = gridDim.x * 8;
+  for (u32 i = blockIdx.x * 8 + (threadIdx.x >> 5); i < nl; i += nwarps) {
+    const int v = longs[i];
+    const long long lo = tc_ld_nc(beg + v);
+    const int d = (int)(tc_ld_nc(beg + v + 1) - lo);
+    const int T = group_slots(d);
+    for (int k = lane; k < T; k += 32) tab[k] = 0;
+    __syncwarp();
+    int nt = 0;
+    for (int k = lane; k < d; k += 32) {
+      const u32 w = rank[tc_ld_nc(adj + lo + k)];
+      if (w >> 4 < (u32)nb) group_insert(tab, T, w);
+      else ++nt;
+    }
+    nt = __reduce_add_sync(TC_FULL_MASK, nt);
+    __syncwarp();
+    const u32 s = row_start(lo, v);
+    int nd = 0;
+    for (int k = lane; k < T; k += 32) nd += tab[k] != 0;
+    nd = __reduce_add_sync(TC_FULL_MASK, nd);
+    const int pad = (nd + 3) & ~3;
+    int put = 0;
+    for (int k = lane; k < T; k += 32) {
+      const u32 e = tab[k];
+      const unsigned bm = __ballot_sync(TC_FULL_MASK, e != 0);
+      if (e) ent[s + entry_place(put + __popc(bm & lt), pad >> 2)] = e;
+      put += __popc(bm);
+    }
+    if (lane < pad - nd) ent[s + entry_place(nd + lane, pad >> 2)] = 0;
+    if (nt) {
+      int at = 0;
+      for (int k0 = 0; k0 < d; k0 += 32) {
+        const u32 w = k0 + lane < d ? rank[tc_ld_nc(adj + lo + k0 + lane)] : 0u;
+        const bool tail = w >> 4 >= (u32)nb;
+        const unsigned bm = __ballot_sync(TC_FULL_MASK, tail);
+        if (tail) ent[s + pad + at + __popc(bm & lt)] = w;
+        at += __popc(bm);
+      }
+    }
+    if (lane == 0) desc[v] = make_int4((int)s, pad, nt, d);
+    __syncwarp();
+  }
+}
+
+// A CTA per longer row (up to BITS_MAX_ROW entries).
+__global__ void __launch_bounds__(512) bits_cta_kernel(const int64_t *__restrict__ beg, const int32_t *__restrict__ adj,
+                                                       int64_t n, const u32 *__restrict__ rank, int nb,
+                                                       u32 *__restrict__ ent, int4 *__restrict__ desc,
+                                                       const int *__restrict__ longs, const u32 *__restrict__ nlongs) {
+  extern __shared__ u32 tab[];
+  __shared__ int wcnt[17];
+  __shared__ int ntail;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lt = tc_lanemask_lt();
+  const u32 nl = nlongs[1];
+  for (u32 i = blockIdx.x; i < nl; i += gridDim.x) {
+    const int v = longs[n - 1 - (int64_t)i];
+    const long long lo = tc_ld_nc(beg + v);
+    const int d = (int)(tc_ld_nc(beg + v + 1) - lo);
+    const int T = group_slots(d);
+    for (int k = threadIdx.x; k < T; k += 512) tab[k] = 0;
+    if (threadIdx.x == 0) ntail = 0;
+    __syncthreads();
+    for (int k = threadIdx.x; k < d; k += 512) {
+      const u32 w = rank[tc_ld_nc(adj + lo + k)];
+      if (w >> 4 < (u32)nb) group_insert(tab, T, w);
+    }
+    __syncthreads();
+    // each warp owns T/16 consecutive slots: count, scan over the warps, write
+    const int seg = T >> 4, k0 = warp * seg;
+    int c = 0;
+    for (int k = lane; k < seg; k += 32) c += tab[k0 + k] != 0;
+    c = __reduce_add_sync(TC_FULL_MASK, c);
+    if (lane == 0) wcnt[warp] = c;
+    __syncthreads();
+    int at = 0, nd = 0;
+    for (int k = 0; k < 16; ++k) {
+      if (k < warp) at += wcnt[k];
+      nd += wcnt[k];
+    }
+    const int pad = (nd + 3) & ~3;
+    const u32 s = row_start(lo, v);
+    for (int k = lane; k < seg; k += 32) {  // seg >= 64
+      const u32 e = tab[k0 + k];
+      const unsigned bm = __ballot_sync(TC_FULL_MASK, e != 0);
+      if (e) ent[s + entry_place(at + __popc(bm & lt), pad >> 2)] = e;
+      at += __popc(bm);
+    }
+    if ((int)threadIdx.x < pad - nd) ent[s + entry_place(nd + threadIdx.x, pad >> 2)] = 0;
+    for (int k = threadIdx.x; k < d; k += 512) {
+      const u32 w = rank[tc_ld_nc(adj + lo + k)];
+      if (w >> 4 >= (u32)nb) ent[s + pad + atomicAdd(&ntail, 1)] = w;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) desc[v] = make_int4((int)s, pad, ntail, d);
+    __syncthreads();  // wcnt, ntail and the table are free again
+  }
+}
+
+// ---- work units ------------------------------------------------------------------------------
+// A table row t (d > table_min) is probed by the rows of its out-neighbours u with d(u) <= d(t)
+// (kept arcs) and of the sources of the arcs moved to it (its in-list).  Its list - out-row, then
+// in-list - is cut into units of about `target` probes.  In-list space is reserved here with one
+// atomic per warp; cur[t] becomes the fill's cursor.
+struct Unit {
+  int t, lo, hi, len_a;
+  u32 a0, b0;
+  int pad0, pad1;
+};
+
+__global__ void __launch_bounds__(256) bits_units_kernel(const int64_t *__restrict__ beg, int64_t n, int64_t row_lo,
+                                                         int64_t row_hi, int table_min, u32 *__restrict__ cnt,
+                                                         const unsigned long long *__restrict__ wsum, u32 *ctr,
+                                                         unsigned long long target, Unit *__restrict__ units) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = tc_lanemask_lt();
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t v0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); v0 < n; v0 += stride) {
+    const int64_t v = v0 + lane;
+    int d = 0;
+    long long b = 0;
+    if (v < n) {
+      b = tc_ld_nc(beg + v);
+      d = (int)(tc_ld_nc(beg + v + 1) - b);
+    }
+    const bool table = d > table_min;
+    if (!__any_sync(TC_FULL_MASK, table)) continue;
+    const u32 nb = table ? cnt[v] : 0u;
+    const int na = table && v >= row_lo && v < row_hi ? d : 0;
+    const u32 len = nb + (u32)na;
+    int k = 0;
+    if (len) {
+      const unsigned long long w = wsum[v];
+      unsigned long long kk = (w + target - 1) / target;
+      kk = max(kk, 1ull);
+      k = (int)min(kk, (unsigned long long)((len + 31) / 32));
+    }
+    // warp-wide exclusive sums of in-list lengths and units
+    u32 sb = nb;
+    int sk = k;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 y = __shfl_up_sync(TC_FULL_MASK, sb, o);
+      const int z = __shfl_up_sync(TC_FULL_MASK, sk, o);
+      if (lane >= o) {
+        sb += y;
+        sk += z;
+      }
+    }
+    u32 ab = 0, ak = 0;
+    if (lane == 31) {
+      if (sb) ab = atomicAdd(ctr + 1, sb);
+      if (sk) ak = atomicAdd(ctr, (u32)sk);
+    }
+    ab = __shfl_sync(TC_FULL_MASK, ab, 31) + sb - nb;
+    ak = __shfl_sync(TC_FULL_MASK, ak, 31) + (u32)(sk - k);
+    if (table) cnt[v] = ab;
+    const u32 per = k ? (len + k - 1) / k : 0;
+    for (int j = 0; j < k; ++j)
+      units[ak + j] = Unit{(int)v, (int)min((u32)j * per, len), (int)min((u32)(j + 1) * per, len), na, (u32)b, ab, 0, 0};
+    (void)lt;
+  }
+}
+
+// In-list fill: every moved arc's source goes to the next free slot of its target's list.
+__global__ void __launch_bounds__(256) bits_fill_kernel(const int2 *__restrict__ pairs,
+                                                        const unsigned long long *__restrict__ npairs,
+                                                        u32 *__restrict__ cur, int32_t *__restrict__ adj_b) {
+  const int64_t np = (int64_t)*npairs;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < np; i += 4 * stride) {
+    int2 p[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) p[r] = i + r * stride < np ? pairs[i + r * stride] : make_int2(-1, 0);
+    u32 slot[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) slot[r] = p[r].x >= 0 ? atomicAdd(cur + p[r].x, 1u) : 0u;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (p[r].x >= 0) adj_b[slot[r]] = p[r].y;
+  }
+}
+
+// ---- counting --------------------------------------------------------------------------------
+constexpr int TAIL_SLOTS = 2048;             // hash slots of a table's tail ids
+constexpr int TAIL_CAP = TAIL_SLOTS / 2;     // tail ids per pass over the unit
+
+__device__ __forceinline__ u32 tail_hash(u32 w) { return w * 0x9E3779B1u >> (32 - 11); }
+
+struct BitsArgs {
+  const int32_t *adj, *adj_b;
+  const int4 *desc;
+  const u32 *ent;
+  const Unit *units;
+  u32 *ctr;  // [0] units, [2] claim head
+  int nb;    // blocks of the bitmap
+  TcControl *ctl;
+};
+
+// Persistent: a CTA claims units and builds the unit's bitmap (plain 16-bit stores: a row has one
+// entry per block).  Its warps claim the list's positions in batches of up to 32 (fewer towards the
+// end of the unit), a lane holding one partner row; the partner ids are loaded two batches ahead
+// and the row descriptors one.  The whole 128-block steps of a row are walked by the warp; what is
+// left of every row (up to four 32-block chunks) goes to a work list in shared memory that the
+// warp's four 8-lane groups drain, so that rows of any length keep the lanes busy.
+// Bound by the shared-memory and load pipe (R-MAT 22 a = 0.70: 71 % busy, 2.8 wavefronts per 16-bit
+// lookup of 32 lanes) and, on graphs whose rows exceed the L2 (R-MAT 22: 19 GB of DRAM reads in
+// 7.3 ms), by the latency of the row loads.  Counting time against the hash tables it replaces: R-MAT
+// 20 ef16 5.7 -> 1.0 ms, R-MAT 24 a = 0.70 163 -> 44 ms.
+__device__ __forceinline__ u32 match4(const unsigned short *tab, uint4 e) {
+  const unsigned char *t = reinterpret_cast<const unsigned char *>(tab);
+  const u32 x0 = *reinterpret_cast<const unsigned short *>(t + (e.x >> 16)) & e.x;
+  const u32 x1 = *reinterpret_cast<const unsigned short *>(t + (e.y >> 16)) & e.y;
+  const u32 x2 = *reinterpret_cast<const unsigned short *>(t + (e.z >> 16)) & e.z;
+  const u32 x3 = *reinterpret_cast<const unsigned short *>(t + (e.w >> 16)) & e.w;
+  return __popc(__byte_perm(x0, x1, 0x5410)) + __popc(__byte_perm(x2, x3, 0x5410));
+}
+
+__device__ __forceinline__ uint4 piece(const uint4 *row, int k, int n) {
+  return k < n ? __ldg(row + k) : make_uint4(0, 0, 0, 0);
+}
+
+__device__ __forceinline__ u32 tail_has(const int *tail, u32 w) {
+  u32 h = tail_hash(w);
+  int x = tail[h];
+  while (x != -1 && x != (int)w) {
+    h = (h + 1) & (TAIL_SLOTS - 1);
+    x = tail[h];
+  }
+  return x == (int)w;
+}
+
+template <int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) bits_count_kernel(BitsArgs p) {
+  constexpr int NW = THREADS / 32;
+  extern __shared__ __align__(16) unsigned char smem[];
+  unsigned short *tab = reinterpret_cast<unsigned short *>(smem);
+  int *tail = reinterpret_cast<int *>(smem + 2 * (size_t)p.nb);
+  __shared__ uint2 rows_all[NW][128];
+  __shared__ Unit su[2];
+  __shared__ int4 sd[2];
+  __shared__ int next_batch;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int gl = lane & 7, grp = lane >> 3;
+  uint2 *rows = rows_all[warp];
+  const unsigned lt = tc_lanemask_lt();
+  const u32 n_units = p.ctr[0];
+  for (int i = threadIdx.x; i < p.nb / 8; i += THREADS) reinterpret_cast<uint4 *>(tab)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = threadIdx.x; i < TAIL_SLOTS; i += THREADS) tail[i] = -1;
+  auto claim = [&](int at) {
+    const u32 x = atomicAdd(p.ctr + 2, 1u);
+    if (x < n_units) {
+      su[at] = p.units[x];
+      sd[at] = p.desc[su[at].t];
+    } else {
+      su[at].t = -1;
+    }
+  };
+  if (threadIdx.x == THREADS - 1) claim(0);
+  unsigned long long hits = 0;
+  for (int cur = 0;; cur ^= 1) {
+    __syncthreads();
+    if (su[cur].t < 0) break;
+    const int lo = su[cur].lo, hi = su[cur].hi, len_a = su[cur].len_a;
+    const int32_t *list_a = p.adj + su[cur].a0, *list_b = p.adj_b + su[cur].b0 - len_a;
+    const int4 td = sd[cur];
+    const u32 ts = (u32)td.x;
+    if (threadIdx.x == THREADS - 1) claim(cur ^ 1);
+    for (int i = threadIdx.x; i < td.y; i += THREADS) {
+      const u32 e = p.ent[ts + i];
+      if (e & 0xffffu) tab[e >> 17] = (unsigned short)e;
+    }
+    for (int t0 = 0; t0 == 0 || t0 < td.z; t0 += TAIL_CAP) {
+      const int tn = min(td.z - t0, TAIL_CAP);
+      for (int i = threadIdx.x; i < tn; i += THREADS) {
+        const int w = (int)p.ent[ts + td.y + t0 + i];
+        u32 h = tail_hash((u32)w);
+        for (int it = 0; it < TAIL_SLOTS && atomicCAS(tail + h, -1, w) != -1; ++it) h = (h + 1) & (TAIL_SLOTS - 1);
+      }
+      if (threadIdx.x == 0) next_batch = lo;
+      __syncthreads();
+      // claim a batch and load its partner ids (-1: no position); ~id on the in-list side
+      auto claim_ids = [&](int &id, bool &in_a) -> bool {
+        int at = 0, bs = 0;
+        if (lane == 0) {
+          bs = min(32, max(4, (hi - *(volatile int *)&next_batch) / (2 * NW)));
+          at = atomicAdd(&next_batch, bs);
+        }
+        at = __shfl_sync(TC_FULL_MASK, at, 0);
+        bs = __shfl_sync(TC_FULL_MASK, bs, 0);
+        id = -1;
+        const int i = at + lane;
+        if (lane < bs && i < hi) {
+          in_a = i < len_a;
+          id = tc_ld_nc((in_a ? list_a : list_b) + i);
+        }
+        return at < hi;
+      };
+      auto fetch = [&](int id, bool in_a) -> int4 {
+        if (id < 0) return make_int4(0, 0, 0, 0);
+        int4 q = __ldg(p.desc + id);
+        if (in_a && q.w > td.w) q = make_int4(0, 0, 0, 0);  // counted from that row's side
+        return q;
+      };
+      u32 acc = 0;
+      int id = -1;
+      bool side = false;
+      bool more = claim_ids(id, side);
+      int4 qn = fetch(id, side);
+      bool later = more && claim_ids(id, side);
+      while (more) {
+        const int4 q = qn;
+        more = later;
+        if (later) {
+          qn = fetch(id, side);
+          later = claim_ids(id, side);
+        }
+        if (t0 == 0) {
+          const int c4 = q.y >> 2;
+          const int rem = c4 & 31;
+          unsigned lm = __ballot_sync(TC_FULL_MASK, c4 >= 32);
+          while (lm) {
+            const int j = __ffs(lm) - 1;
+            lm &= lm - 1;
+            const uint4 *r = reinterpret_cast<const uint4 *>(p.ent + (u32)__shfl_sync(TC_FULL_MASK, q.x, j)) + lane;
+            int steps = __shfl_sync(TC_FULL_MASK, c4, j) >> 5;
+            for (; steps >= 2; steps -= 2, r += 64) {
+              const uint4 e0 = __ldg(r), e1 = __ldg(r + 32);
+              acc += match4(tab, e0) + match4(tab, e1);
+            }
+            if (steps) acc += match4(tab, __ldg(r));
+          }
+          const int nch = (rem + 7) >> 3;  // 0..4
+          const unsigned b0 = __ballot_sync(TC_FULL_MASK, nch & 1), b1 = __ballot_sync(TC_FULL_MASK, nch & 2),
+                         b2 = __ballot_sync(TC_FULL_MASK, nch & 4);
+          const int n = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+          if (n) {
+            const int at = __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
+            const u32 s = (u32)q.x + 4u * (u32)(c4 - rem);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (j < nch) rows[at + j] = make_uint2(s + 32u * j, (u32)(rem - 8 * j));
+            __syncwarp();
+            for (int i = grp; i - grp < n; i += 8) {
+              const uint2 ra = i < n ? rows[i] : make_uint2(0, 0), rb = i + 4 < n ? rows[i + 4] : make_uint2(0, 0);
+              const uint4 ea = piece(reinterpret_cast<const uint4 *>(p.ent + ra.x), gl, (int)ra.y);
+              const uint4 eb = piece(reinterpret_cast<const uint4 *>(p.ent + rb.x), gl, (int)rb.y);
+              acc += match4(tab, ea) + match4(tab, eb);
+            }
+            __syncwarp();
+          }
+        }
+        if (tn > 0) {  // tail ids against the hash set
+          const unsigned km = __ballot_sync(TC_FULL_MASK, q.z > 0);
+          const int n = __popc(km);
+          if (n) {
+            if (q.z > 0) rows[__popc(km & lt)] = make_uint2((u32)(q.x + q.y), (u32)q.z);
+            __syncwarp();
+            for (int i = 0; i < n; i += 8) {
+              const uint2 ra = i + grp < n ? rows[i + grp] : make_uint2(0, 0);
+              const uint2 rb = i + 4 + grp < n ? rows[i + 4 + grp] : make_uint2(0, 0);
+              const int nm = __reduce_max_sync(TC_FULL_MASK, max((int)ra.y, (int)rb.y));
+              for (int k = gl; k - gl < nm; k += 8) {
+                const bool va = k < (int)ra.y, vb = k < (int)rb.y;
+                const u32 wa = va ? __ldg(p.ent + ra.x + k) : 0u, wb = vb ? __ldg(p.ent + rb.x + k) : 0u;
+                if (va) acc += tail_has(tail, wa);
+                if (vb) acc += tail_has(tail, wb);
+              }
+            }
+            __syncwarp();
+          }
+        }
+      }
+      hits += acc;
+      __syncthreads();
+      if (tn > 0) {
+        for (int i = threadIdx.x; i < TAIL_SLOTS; i += THREADS) tail[i] = -1;
+        __syncthreads();
+      }
+    }
+    for (int i = threadIdx.x; i < td.y; i += THREADS) {
+      const u32 e = p.ent[ts + i];
+      if (e & 0xffffu) tab[e >> 17] = 0;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) hits += __shfl_down_sync(TC_FULL_MASK, hits, o);
+  if (lane == 0 && hits) atomicAdd(&p.ctl->count, hits);
+}
+
+// 256 threads, five CTAs per SM.  Measured on R-MAT 22 / R-MAT 25 ef32 (call, ms): 512 threads x 3
+// 15.7 / 538, 256 x 5 12.3 / 423, 256 x 6 with 40 registers 12.5 / 432, 256 x 4 13.0 / 456; the bitmap
+// of 8192, 13,312, 16,384 (four CTAs) blocks 12.3 / 423, 12.3 / 415, 12.8 / 427.
+constexpr int BITS_THREADS = 256;
+constexpr int BITS_MINB = 5;
+constexpr int BITS_MAX_BLOCKS = 13312;  // bitmap of 212,992 columns, 26 KiB; at most 32,767 (entry format)
+
+int blocks_for(int64_t work, int64_t per, int num_sms, int most_per_sm) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>((work + per - 1) / per, (int64_t)num_sms * most_per_sm));
+}
+
+}  // namespace
+
+bool bits_eligible(const DevGraph3 &g, int64_t max_out_degree) {
+  return max_out_degree > BITS_TABLE_MIN && max_out_degree <= BITS_MAX_ROW && g.mA + 6 * g.rows + 8 < ((int64_t)1 << 32);
+}
+
+// Enqueue the conversion and the work units (after the scheduling pass and its readback).
+int bits_prepare(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, int64_t row_lo,
+                 int64_t row_hi, const SchedPlan &plan, int64_t max_out_degree, cudaStream_t st, BitsPlan *out) {
+  const int nb = (int)std::min<int64_t>((((n + 15) / 16) + 7) & ~7ll, BITS_MAX_BLOCKS);
+  const u32 ntiles = (u32)((n + RK_TILE - 1) / RK_TILE);
+  // units: every table at least one, and one more per `target` probes: about eight units per resident
+  // CTA, so the last ones end together, but not so small that a unit's set-up shows (R-MAT 18: 1.63 ms
+  // at 2^18 probes, 1.81 at 2^20; R-MAT 25: 426 and 415)
+  const unsigned long long target = std::min<unsigned long long>(
+      std::max<unsigned long long>(plan.w_min / (unsigned long long)(c->num_sms * BITS_MINB * 8), 1ull << 16), 1ull << 20);
+  const int64_t max_units = m / (BITS_TABLE_MIN + 1) + (int64_t)(plan.w_min / target) + 1;
+  // one scratch block: in-degrees, ranks, rank histogram, counters, row lists
+  const size_t nn = (size_t)n;
+  const size_t hist = 256 * (size_t)ntiles;
+  int rc;
+  if ((rc = ensure((void **)&c->d_bits_cols, &c->bits_cols_cap,
+                   sizeof(u32) * (3 * nn + hist + scan_u32_scratch(256 * (int64_t)ntiles) + 16))))
+    return rc;
+  if ((rc = ensure((void **)&c->d_bits_desc, &c->bits_desc_cap, sizeof(int4) * nn))) return rc;
+  if ((rc = ensure((void **)&c->d_bits_ent, &c->bits_ent_cap, sizeof(u32) * (size_t)(m + 6 * n + 8)))) return rc;
+  if ((rc = ensure((void **)&c->d_bits_units, &c->bits_units_cap, sizeof(Unit) * (size_t)max_units))) return rc;
+  if ((rc = ensure((void **)&c->d_split_adj, &c->split_adj_cap, sizeof(int32_t) * (size_t)std::max<int64_t>(m, 1))))
+    return rc;
+  u32 *indeg = c->d_bits_cols, *rank = indeg + nn, *counts = rank + nn;
+  u32 *scratch = counts + hist;
+  u32 *ctr = scratch + scan_u32_scratch(256 * (int64_t)ntiles);  // units, in-list entries, claims, warp rows, CTA rows
+  int *longs = reinterpret_cast<int *>(ctr + 16);
+  int4 *desc = reinterpret_cast<int4 *>(c->d_bits_desc);
+  Unit *units = reinterpret_cast<Unit *>(c->d_bits_units);
+  TC_CUDA_TRY(cudaMemsetAsync(indeg, 0, sizeof(u32) * nn, st));
+  TC_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(u32) * 16, st));
+  indeg_kernel<<<blocks_for(m, 1024, c->num_sms, 16), 256, 0, st>>>(adj, m, indeg);
+  rank_hist_kernel<<<ntiles, 256, 0, st>>>(indeg, n, counts, ntiles);
+  TC_CUDA_TRY(cudaGetLastError());
+  note_launch(2);
+  if ((rc = scan_exclusive_u32(counts, counts, 256 * (int64_t)ntiles, scratch, st))) return rc;
+  rank_scatter_kernel<<<ntiles, 256, 0, st>>>(indeg, n, counts, ntiles, rank);
+  bits_short_kernel<<<blocks_for(n, 256, c->num_sms, 32), 256, 0, st>>>(beg, adj, n, rank, nb, c->d_bits_ent, desc,
+                                                                        longs, ctr + 3);
+  bits_warp_kernel<<<c->num_sms * 7, 256, 0, st>>>(beg, adj, rank, nb, c->d_bits_ent, desc, longs, ctr + 3);
+  note_launch(3);
+  TC_CUDA_TRY(cudaGetLastError());
+  if (max_out_degree > BITS_WARP_ROW) {
+    int T = 64;
+    while (T < 2 * max_out_degree) T <<= 1;
+    const int smem = 4 * T;
+    TC_CUDA_TRY(cudaFuncSetAttribute(bits_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 2 * BITS_MAX_ROW));
+    bits_cta_kernel<<<c->num_sms * std::min(4, (int)(200 * 1024 / (smem + 2048))), 512, smem, st>>>(
+        beg, adj, n, rank, nb, c->d_bits_ent, desc, longs, ctr + 3);
+    note_launch();
+    TC_CUDA_TRY(cudaGetLastError());
+  }
+  bits_units_kernel<<<blocks_for(n, 256, c->num_sms, 16), 256, 0, st>>>(beg, n, row_lo, row_hi, BITS_TABLE_MIN,
+                                                                        c->d_split_cnt, c->d_split_wsum, ctr, target,
+                                                                        units);
+  bits_fill_kernel<<<blocks_for(m, 256, c->num_sms, 16), 256, 0, st>>>(c->d_split_pairs, c->d_split_plans + 4,
+                                                                       c->d_split_cnt, c->d_split_adj);
+  note_launch(2);
+  TC_CUDA_TRY(cudaGetLastError());
+  out->nb = nb;
+  out->ctr = ctr;
+  return TRUST_TC_OK;
+}
+
+int bits_launch(trust_tc_ctx *c, const BitsPlan &plan, const int32_t *adj, TcControl *ctl, cudaStream_t st) {
+  BitsArgs a{};
+  a.adj = adj;
+  a.adj_b = c->d_split_adj;
+  a.desc = reinterpret_cast<const int4 *>(c->d_bits_desc);
+  a.ent = c->d_bits_ent;
+  a.units = reinterpret_cast<const Unit *>(c->d_bits_units);
+  a.ctr = plan.ctr;
+  a.nb = plan.nb;
+  a.ctl = ctl;
+  const auto kernel = bits_count_kernel<BITS_THREADS, BITS_MINB>;
+  const size_t smem = 2 * (size_t)plan.nb + 4 * TAIL_SLOTS;
+  TC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   2 * BITS_MAX_BLOCKS + 4 * TAIL_SLOTS));
+  TC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  int per_sm = 0;
+  TC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, BITS_THREADS, smem));
+  kernel<<<c->num_sms * std::max(per_sm, 1), BITS_THREADS, smem, st>>>(a);
+  note_launch();
+  TC_CUDA_TRY(cudaGetLastError());
+  return TRUST_TC_OK;
+}
+
+}  // namespace tc

@@ -825,7 +825,7 @@ __device__ __forceinline__ void cta_arcs(const CountArgs &p, const Set &set, int
     const int i = (bt << 5) + lane;
     int s = 0, dd = 0;
     if (i < dB) row_of(p.begC, tc_ld_nc(p.adjB + bB + i), s, dd);
-    if (p.split && dd > dA) dd = 0;
+    if (p.split && dd > max(dA, p.table_min)) dd = 0;
     if (longs) {
       const bool lg = dd >= TC_CTA_LONG;
       const unsigned lm = __ballot_sync(TC_FULL_MASK, lg);
@@ -924,7 +924,7 @@ __device__ __forceinline__ void warp_vertex(const CountArgs &p, int v, int *warp
     const int i = a0 + lane;
     int s = 0, dd = 0;
     if (i < dB) row_of(p.begC, tc_ld_nc(p.adjB + bB + i), s, dd);
-    if (p.split && dd > dA) dd = 0;
+    if (p.split && dd > max(dA, p.table_min)) dd = 0;
     probe_arcs<32, LongRow<32>::value>(p.adjC, s, dd, lane, set, hits, wedges);
   }
   __syncwarp();
@@ -994,7 +994,7 @@ __device__ void drain_group_class(const CountArgs &p, int c, int *warp_tab, unsi
   auto ld_target = [&](GroupStage &x) {
     x.s = 0; x.dd = 0;
     if (x.uB >= 0) row_of(p.begC, x.uB, x.s, x.dd);
-    if (p.split && x.dd > x.d) x.dd = 0;  // counted from u's side in the second pass
+    if (p.split && x.dd > max(x.d, p.table_min)) x.dd = 0;  // counted from u's side in the second pass
   };
   for (;;) {
     int t0 = 0;
@@ -1071,7 +1071,7 @@ __global__ void __launch_bounds__(MAXT, MINB) count_kernel(CountArgs p) {
   // Phase A: CTA-granularity vertices, largest class first.
   for (int c = TC_CLASS_HUGE; c >= TC_CLASS_CTA; --c) {
     const int n_items = p.ctl->class_count[c];
-    if (n_items == 0) continue;
+    if (n_items == 0 || (c == TC_CLASS_HUGE && p.table_min > 0)) continue;
     if (c == TC_CLASS_HUGE && (int)blockIdx.x >= p.huge_blocks) continue;
     const int *list = class_list_t<BATCH>(p, c);
     int *tab = (c == TC_CLASS_HUGE) ? p.huge_tables + (size_t)blockIdx.x * ((size_t)1 << p.huge_log2)
@@ -1087,6 +1087,11 @@ __global__ void __launch_bounds__(MAXT, MINB) count_kernel(CountArgs p) {
         int hb, hd;
         row_of(p.begA, arow(p, v), hb, hd);
         if (hd <= p.hub_max_degree) continue;
+      }
+      if (p.table_min > 0) {
+        int b, d;
+        row_of(p.begA, arow(p, v), b, d);
+        if (d > p.table_min) continue;
       }
       const long long t_start = REC ? clock64() : 0;
       const unsigned long long h0 = hits;
@@ -1113,6 +1118,11 @@ __global__ void __launch_bounds__(MAXT, MINB) count_kernel(CountArgs p) {
       const int t1 = min(t0 + claim, n_items);
       for (int t = t0; t < t1; ++t) {
         const int v = list[t];
+        if (p.table_min > 0) {
+          int b, d;
+          row_of(p.begA, arow(p, v), b, d);
+          if (d > p.table_min) continue;
+        }
         const long long t_start = REC ? clock64() : 0;
         const unsigned long long h0 = hits;
         warp_vertex<SAME>(p, v, warp_tab, hits, wedges);
@@ -1359,7 +1369,7 @@ __global__ void __launch_bounds__(512, 2) hub_kernel(CountArgs p, int log2C, int
         const int i = (bt << 5) + lane;
         int s = 0, dd = 0;
         if (i < dB) row_of(p.begC, tc_ld_nc(p.adjB + bB + i), s, dd);
-        if (p.split && dd > dA) dd = 0;
+        if (p.split && dd > max(dA, p.table_min)) dd = 0;
         probe_arcs<32, LongRow<32>::value>(p.adjC, s, dd, lane, tset, hits, wedges);
       }
     };

@@ -47,6 +47,10 @@ struct CountArgs {
   // quotient tables), and the CTA table may use cta_table_bytes of dynamic shared memory
   int key_bits;
   int cta_table_bytes;
+  // > 0: rows longer than this, and with split the arcs to them, are counted elsewhere (the
+  // block-bitmap path): such rows are passed over, and an arc is left out when
+  // d(u) > max(d(v), table_min)
+  int table_min;
 };
 
 int launch_check(const int64_t *beg, const int32_t *adj, int64_t rows, int64_t m, int64_t id_bound,

@@ -51,6 +51,14 @@ struct trust_tc_ctx {
   size_t split_rowmap_cap = 0;
   int32_t *d_split_adj = nullptr;
   size_t split_adj_cap = 0;
+  unsigned *d_bits_cols = nullptr;  // block-bitmap path: column popularity and ranks, counters, row lists
+  size_t bits_cols_cap = 0;
+  unsigned *d_bits_ent = nullptr;  // every row as block entries, then tail ids
+  size_t bits_ent_cap = 0;
+  int4 *d_bits_desc = nullptr;  // per row: first entry, block entries, tail ids, out-degree
+  size_t bits_desc_cap = 0;
+  void *d_bits_units = nullptr;  // work units
+  size_t bits_units_cap = 0;
   int64_t *d_beg = nullptr;
   size_t beg_cap = 0;
   int32_t *d_adj = nullptr;
@@ -104,6 +112,9 @@ void ctx_release(trust_tc_ctx *c);
 int ensure(void **p, size_t *cap, size_t bytes);
 int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bool check_ids,
                  trust_tc_result *r);
+// Exclusive u32 scan (in may equal out) with caller-provided scratch of scan_u32_scratch(n) words.
+size_t scan_u32_scratch(int64_t n);
+int scan_exclusive_u32(const unsigned *in, unsigned *out, int64_t n, unsigned *scratch, cudaStream_t st);
 int scan_exclusive_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t st, int64_t *total);
 // The n x n hash partition of a device CSR into p*p tiles (tile i*p+j) in pinned host memory
 // (free each beg / adj with cudaFreeHost); p <= 32.
@@ -121,10 +132,12 @@ struct SchedPlan {
   int64_t moved_arcs;               // pair slots the pass used (moved arcs and holes)
   bool overflow;                    // the pair arrays ran out (never expected): no split
 };
-// Only source rows in [row_lo, row_hi) are walked (their arcs planned and moved).
+// Only source rows in [row_lo, row_hi) are walked (their arcs planned and moved).  An arc (v,u) is
+// moved to u's side when d(u) > max(d(v), table_min); with table_min > 0 the work sum of a row
+// longer than table_min also holds the probes of the arcs it keeps.
 int split_plan(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, cudaStream_t st,
                const float *d_model, int warp_max, int cta_max, float promote_log2, int cta_warps, TcControl *ctl,
-               int64_t row_lo, int64_t row_hi);
+               int64_t row_lo, int64_t row_hi, int table_min);
 // after the stream has synchronised
 void split_plan_read(const trust_tc_ctx *c, SchedPlan *plan);
 int radix_sort_u64(unsigned long long *keys, unsigned long long *tmp, int64_t n, const int *shifts, int nshifts,

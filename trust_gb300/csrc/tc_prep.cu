@@ -119,6 +119,28 @@ static int scan_exclusive(const T *in, T *out, int64_t n, cudaStream_t st, T *to
   return TRUST_TC_OK;
 }
 
+size_t scan_u32_scratch(int64_t n) {
+  size_t words = 0;
+  for (int64_t nb = (n + RS_TILE - 1) / RS_TILE; nb > 1; nb = (nb + RS_TILE - 1) / RS_TILE) words += (size_t)nb;
+  return words;
+}
+
+int scan_exclusive_u32(const unsigned *in, unsigned *out, int64_t n, unsigned *scratch, cudaStream_t st) {
+  if (n <= 0) return TRUST_TC_OK;
+  const int64_t nb = (n + RS_TILE - 1) / RS_TILE;
+  if (nb > 1) {
+    scan_reduce_kernel<u32><<<(unsigned)nb, RS_THREADS, 0, st>>>(in, n, scratch);
+    TC_NOTE_LAUNCH();
+    TC_CUDA_TRY(cudaGetLastError());
+    int rc = scan_exclusive_u32(scratch, scratch, nb, scratch + nb, st);
+    if (rc) return rc;
+  }
+  scan_down_kernel<u32><<<(unsigned)nb, RS_THREADS, 0, st>>>(in, out, n, nb > 1 ? scratch : nullptr);
+  TC_NOTE_LAUNCH();
+  TC_CUDA_TRY(cudaGetLastError());
+  return TRUST_TC_OK;
+}
+
 int scan_exclusive_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t st, int64_t *total) {
   return scan_exclusive<int64_t>(in, out, n, st, total);
 }

@@ -277,7 +277,7 @@ __global__ void sched_short_kernel(const int64_t *__restrict__ beg, const int32_
                                    int64_t row_lo, int64_t row_hi, unsigned *__restrict__ cnt,
                                    unsigned long long *__restrict__ wsum, unsigned long long *plans,
                                    int *__restrict__ longs, int2 *__restrict__ pairs, unsigned long long pair_cap,
-                                   TcControl *ctl) {
+                                   int table_min, TcControl *ctl) {
   const int lane = threadIdx.x & 31;
   unsigned long long w_all = 0, w_min = 0;
   int bad = 0;
@@ -291,7 +291,7 @@ __global__ void sched_short_kernel(const int64_t *__restrict__ beg, const int32_
                  w_min += (unsigned)min(du, dv);
                  if (!last) bad |= u >= tc_ld_nc(adj + pos + 1);
                }
-               move_arc(valid && du > dv, u, v, dv, cnt, wsum, pairs, plans + PLAN_NPAIRS, pb);
+               move_arc(valid && du > max(dv, table_min), u, v, dv, cnt, wsum, pairs, plans + PLAN_NPAIRS, pb);
              });
   pair_holes(pb, pairs);
 #pragma unroll
@@ -318,7 +318,7 @@ __global__ void sched_long_kernel(const int64_t *__restrict__ beg, const int32_t
                                   const float *__restrict__ model, int warp_max, int cta_max, float promote_log2,
                                   unsigned char *__restrict__ dec, float *__restrict__ pred, float *sums,
                                   int cta_warps, int2 *__restrict__ pairs, unsigned long long pair_cap,
-                                  TcControl *ctl) {
+                                  int table_min, TcControl *ctl) {
   __shared__ float P[MODEL ? TC_MODEL_FLOATS : 1];
   if (MODEL) {  // staged with W1 and W2 transposed (see warp_mlp)
     for (int i = threadIdx.x; i < TC_MODEL_FLOATS; i += blockDim.x) {
@@ -352,12 +352,12 @@ __global__ void sched_long_kernel(const int64_t *__restrict__ beg, const int32_t
     unsigned long long rw = 0, rmin = 0;
     int rmax = 0, rnb = 0;
     long_row_arcs(beg, adj, (int)lo, dv, lane, [&](bool valid, int u, int du, int pos, bool last) {
-      const bool mv = valid && du > dv;
+      const bool mv = valid && du > max(dv, table_min);
       if (valid) {
         rw += (unsigned)du;
         rmin += (unsigned)min(du, dv);
         rmax = max(rmax, du);
-        rnb += mv;
+        rnb += du > dv;
         if (!last) bad |= u >= tc_ld_nc(adj + pos + 1);
       }
       move_arc(mv, u, v, dv, cnt, wsum, pairs, plans + PLAN_NPAIRS, pb);
@@ -372,6 +372,8 @@ __global__ void sched_long_kernel(const int64_t *__restrict__ beg, const int32_t
     if (lane == 0) {
       w_all += rw;
       w_min += rmin;
+      if (table_min && dv > table_min)  // probes of the arcs the row keeps
+        atomicAdd(wsum + v, rmin - (unsigned long long)rnb * (unsigned)dv);
     }
     if (MODEL) {
       const int cls = tuned_class_of(dv, warp_max, cta_max);
@@ -459,7 +461,7 @@ static size_t pair_slots(int64_t arcs, int64_t warps) {
 // the totals reach the host with the stream's next synchronisation (split_plan_read).
 int split_plan(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, cudaStream_t st,
                const float *d_model, int warp_max, int cta_max, float promote_log2, int cta_warps, TcControl *ctl,
-               int64_t row_lo, int64_t row_hi) {
+               int64_t row_lo, int64_t row_hi, int table_min) {
   const size_t nn = (size_t)std::max<int64_t>(n + 1, 1);
   int rc = ensure((void **)&c->d_split_cnt, &c->split_cnt_cap, sizeof(unsigned) * nn);
   if (rc) return rc;
@@ -480,17 +482,17 @@ int split_plan(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t 
   float *sums = reinterpret_cast<float *>(c->d_split_plans + PLAN_SAVED);
   if (row_hi <= 0) row_hi = n;
   sched_short_kernel<<<sb, 256, 0, st>>>(beg, adj, n, row_lo, row_hi, c->d_split_cnt, c->d_split_wsum,
-                                         c->d_split_plans, c->d_sched_long, c->d_split_pairs, slots, ctl);
+                                         c->d_split_plans, c->d_sched_long, c->d_split_pairs, slots, table_min, ctl);
   TC_NOTE_LAUNCH();
   TC_CUDA_TRY(cudaGetLastError());
   if (d_model)
     sched_long_kernel<true><<<lb, 256, 0, st>>>(beg, adj, c->d_split_cnt, c->d_split_wsum, c->d_split_plans,
                                                 c->d_sched_long, d_model, warp_max, cta_max, promote_log2, c->d_dec,
-                                                c->d_pred, sums, cta_warps, c->d_split_pairs, slots, ctl);
+                                                c->d_pred, sums, cta_warps, c->d_split_pairs, slots, table_min, ctl);
   else
     sched_long_kernel<false><<<lb, 256, 0, st>>>(beg, adj, c->d_split_cnt, c->d_split_wsum, c->d_split_plans,
                                                  c->d_sched_long, nullptr, warp_max, cta_max, promote_log2, nullptr,
-                                                 nullptr, nullptr, cta_warps, c->d_split_pairs, slots, ctl);
+                                                 nullptr, nullptr, cta_warps, c->d_split_pairs, slots, table_min, ctl);
   TC_NOTE_LAUNCH();
   TC_CUDA_TRY(cudaGetLastError());
   TC_CUDA_TRY(cudaMemcpyAsync(c->h_plans, c->d_split_plans, TC_PLAN_WORDS * sizeof(unsigned long long),
