@@ -140,8 +140,6 @@ int split_plan(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t 
                int64_t row_lo, int64_t row_hi, int table_min);
 // after the stream has synchronised
 void split_plan_read(const trust_tc_ctx *c, SchedPlan *plan);
-int radix_sort_u64(unsigned long long *keys, unsigned long long *tmp, int64_t n, const int *shifts, int nshifts,
-                   cudaStream_t st);
 // heaviest first: reorder the list of each of the given classes by predicted cycles, descending
 int lpt_sort(trust_tc_ctx *c, int *lists, const int *off, const int *counts, const float *pred, cudaStream_t st);
 int vertex_features(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t n, int warp_max,
