@@ -1,0 +1,90 @@
+"""The one-launch path for small graphs (tc_small.cu) against the oracle: any CSR (unsorted rows,
+duplicates, self-loops), its size bounds, dense graphs whose rows are shared by several warps, row
+ranges, and invalid input at every position."""
+import numpy as np
+import pytest
+
+import trust_gb300 as T
+from trust_gb300 import _lib
+from oracle import oracle as O
+from tests import graphs
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _dev(beg, adj):
+    return (torch.from_numpy(np.ascontiguousarray(beg, dtype=np.int64)).cuda(),
+            torch.from_numpy(np.ascontiguousarray(adj, dtype=np.int32)).cuda())
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    with T.Context() as c:
+        yield c
+
+
+def _same_as_general(ctx, beg, adj, expect):
+    db, da = _dev(beg, adj)
+    r = T.count_csr(db, da, ctx=ctx)
+    g = T.count_csr(db, da, ctx=ctx, chunk=8)  # a launch parameter: the general path
+    assert r.triangles == g.triangles == expect
+    assert (r.wedges, r.max_out_degree, r.class_sizes) == (g.wedges, g.max_out_degree, g.class_sizes)
+    assert r.wedges == O.wedges(beg, adj)
+    h = T.count_csr(beg, adj, ctx=ctx)  # host input
+    assert h.triangles == expect
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 65, 500])
+@pytest.mark.parametrize("max_deg", [1, 3, 32, 33, 200])
+def test_any_csr(ctx, n, max_deg):
+    rng = np.random.default_rng(n * 1000 + max_deg)
+    for _ in range(3):
+        beg, adj = graphs.random_csr(rng, n, max_deg)
+        _same_as_general(ctx, beg, adj, O.count_forward(beg, adj))
+
+
+@pytest.mark.parametrize("n", [65_535, 65_536, 65_537])
+@pytest.mark.parametrize("m", [100_000, (1 << 21) - 1, 1 << 21])
+def test_size_bounds(ctx, n, m):
+    rng = np.random.default_rng(n + m)
+    d = rng.multinomial(m, np.full(n, 1 / n))
+    beg = np.concatenate([[0], np.cumsum(d)]).astype(np.int64)
+    adj = rng.integers(0, n, size=m).astype(np.int32)
+    adj[rng.random(m) < 0.2] = n - 1
+    _same_as_general(ctx, beg, adj, O.count_forward(beg, adj, threads=8))
+
+
+@pytest.mark.parametrize("n", [40, 130, 300, 600])
+def test_dense(ctx, n):
+    pairs, tri = graphs.complete(n)
+    beg, adj = O.build_csr(pairs, n)
+    _same_as_general(ctx, beg, adj, tri)
+    whole = 0
+    for lo, hi in ((0, 1), (1, n // 3), (n // 3, n)):
+        r = T.count_csr(*_dev(beg, adj), ctx=ctx, row_range=(lo, hi))
+        assert r.triangles == O.count_forward_sorted_range(beg, adj, lo, hi, 2, 1)
+        whole += r.triangles
+    assert whole == tri
+
+
+def test_invalid_input(ctx):
+    rng = np.random.default_rng(2)
+    n = 300
+    beg, adj = graphs.random_csr(rng, n, 60, 0, 0)
+    expect = O.count_forward(beg, adj)
+    for pos in (0, 1, 31, 32, adj.size // 2, adj.size - 1):
+        for bad in (-1, n, 2**31 - 1):
+            a = adj.copy()
+            a[pos] = bad
+            with pytest.raises(T.TrustTcError) as e:
+                T.count_csr(*_dev(beg, a), ctx=ctx)
+            assert e.value.status == _lib.E_IDS
+            assert T.count_csr(*_dev(beg, adj), ctx=ctx).triangles == expect  # the context is clean again
+    for pos, val in ((0, 1), (1, -5), (n // 2, 2**40), (n // 2, -(2**40)), (n, adj.size - 1), (n, adj.size + 1)):
+        b = beg.copy()
+        b[pos] = val
+        with pytest.raises(T.TrustTcError) as e:
+            T.count_csr(*_dev(b, adj), ctx=ctx)
+        assert e.value.status == _lib.E_OFFSETS
+        assert T.count_csr(*_dev(beg, adj), ctx=ctx).triangles == expect

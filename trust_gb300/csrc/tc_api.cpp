@@ -22,6 +22,7 @@
 #include "tc_count.h"
 #include "tc_internal.h"
 #include "tc_model.h"
+#include "tc_small.h"
 
 namespace tc {
 
@@ -105,6 +106,7 @@ void ctx_release(trust_tc_ctx *c) {
   cudaFree(c->d_split_cbeg);
   cudaFree(c->d_split_rowmap);
   cudaFree(c->d_split_adj);
+  cudaFree(c->d_small);
   cudaFree(c->d_bits_cols);
   cudaFree(c->d_bits_ent);
   cudaFree(c->d_bits_desc);
@@ -240,6 +242,32 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
   // source rows whose arcs are counted (one CSR): [row_lo, row_hi); row_hi = -1 means all rows
   const int64_t row_lo = g.row_lo, row_hi = g.row_hi > 0 ? g.row_hi : -1;
   TC_CUDA_TRY(cudaEventRecord(c->ev[0], st));
+  // a small graph under the default schedule and launch shape: everything in one launch (the direction
+  // split, cycle recording and the hub kernel's own options keep the general path)
+  const bool defaults = o.schedule == TRUST_TC_SCHED_LEARNED && o.direction_split != 1 && !o.record_cycles &&
+                        o.threads_per_block <= 0 && o.blocks <= 0 && o.chunk <= 0 && o.warp_max_degree <= 0 &&
+                        o.block_max_degree <= 0 && o.hub_cluster == 0 && !o.test_wait_expiry;
+  if (defaults && same && !g.rowmap && g.min_deg == 2 && small_graph(g.rows, g.mA)) {
+    rc = small_count(c, g.begA, g.adjA, g.rows, g.mA, row_lo, row_hi < 0 ? g.rows : row_hi, check_ids, cfg.warp_max,
+                     cfg.cta_max, st);
+    if (rc) return rc;
+    TC_CUDA_TRY(cudaEventRecord(c->ev[4], st));
+    TC_CUDA_TRY(cudaStreamSynchronize(st));
+    const TcControl &h = *c->h_ctl;
+    if (h.status & TC_DEV_BAD_OFFSETS) return TRUST_TC_E_OFFSETS;
+    if (h.status & TC_DEV_BAD_IDS) return TRUST_TC_E_IDS;
+    float ms = 0;
+    TC_CUDA_TRY(cudaEventElapsedTime(&ms, c->ev[0], c->ev[4]));
+    r->triangles = h.count;
+    r->wedges = (int64_t)h.wedges;
+    r->kernel_seconds = r->count_seconds = r->call_seconds = ms * 1e-3;
+    r->max_out_degree = h.max_out_degree;
+    const bool plain = h.max_out_degree >= TC_SMALL_SKEWED_MIN_ROW;  // as the general path chooses
+    for (int k = 0; k < TC_NUM_CLASSES; ++k) r->class_sizes[k] = plain ? h.class_count_alt[k] : h.class_count[k];
+    r->direction_split = 0;
+    r->split_saving_ms = 0.f;
+    return TRUST_TC_OK;
+  }
   TC_CUDA_TRY(cudaMemsetAsync(ctl, 0, sizeof(TcControl), st));
   ListOffsets off{};
   // one CSR: validation, class histogram and list scatter in one kernel, each class listed in a

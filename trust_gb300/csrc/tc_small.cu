@@ -1,0 +1,220 @@
+// tc_small.cu — graphs small enough that latency is the whole cost: one launch, one synchronisation.
+//
+// The general path checks and classifies the rows, reads the class sizes back, launches the counting
+// kernel over five class queues and reads the count back: two host round trips and about thirty
+// dependent memory latencies around a few microseconds of work.  Here one kernel does all of it: a
+// warp per (row, every S-th batch of 32 arcs) checks what it reads before using it as an index,
+// builds the row's bitmap over all ids in shared memory (a probe is one 4-byte load, no hashing) and
+// probes it, four rows at a time, eight lanes each; the last CTA to finish writes the totals
+// straight into the context's pinned control block and clears the accumulators.
+// Calls on GB300, general path / this one, us: R-MAT 8 (1,311 arcs) 79 / 28, R-MAT 16 ef16 (0.9 M)
+// 404 / 162, K_512 191 / 79, Erdos-Renyi 60,000 / 1.9 M arcs 161 / 133, one row of 15,000 entries 828
+// / 555.  Small graphs are bound by the launch and the round trip (device time 12 of R-MAT 8's 28 us),
+// R-MAT 16 by the issue of its 94 M probes and the tail of its longest rows.
+#include <algorithm>
+
+#include "tc_count.h"
+#include "tc_internal.h"
+#include "tc_small.h"
+
+namespace tc {
+
+namespace {
+
+constexpr int SM_WARPS = 8;
+constexpr int SM_THREADS = 32 * SM_WARPS;
+
+struct SmallArgs {
+  const int64_t *beg;
+  const int32_t *adj;
+  int n, m;
+  int row_lo, row_hi;
+  int check_ids;
+  int warp_max, cta_max;
+  int splits;   // warps per row
+  int words;    // bitmap words per warp
+  TcControl *acc;    // device accumulators, zero between calls (bad_offset_at: CTAs finished)
+  TcControl *out;    // pinned host block
+};
+
+// A row that may be indexed: begin <= end inside the arc array.  Rows out of bounds are reported by
+// the warp that owns them.
+__device__ __forceinline__ int checked_row(const SmallArgs &p, int v, int &b) {
+  const long long lo = tc_ld_nc(p.beg + v), hi = tc_ld_nc(p.beg + v + 1);
+  b = (int)lo;
+  if (lo < 0 || hi < lo || hi > p.m) return -1;
+  return (int)(hi - lo);
+}
+
+__global__ void __launch_bounds__(SM_THREADS, 6) small_kernel(SmallArgs p) {
+  extern __shared__ unsigned bitmaps[];
+  __shared__ int hist[2][TC_NUM_CLASSES];
+  __shared__ unsigned long long s_count, s_wedges;
+  __shared__ int s_bad, s_dmax, s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int grp = lane >> 3, gl = lane & 7;
+  unsigned *words = bitmaps + warp * p.words;
+  for (int i = lane; i < p.words; i += 32) words[i] = 0;
+  if (threadIdx.x < 2 * TC_NUM_CLASSES) (&hist[0][0])[threadIdx.x] = 0;
+  if (threadIdx.x == 0) {
+    s_count = s_wedges = 0;
+    s_bad = s_dmax = 0;
+    if (blockIdx.x == 0 && (tc_ld_nc(p.beg) != 0 || tc_ld_nc(p.beg + p.n) != p.m)) s_bad = TC_DEV_BAD_OFFSETS;
+  }
+  __syncthreads();
+  unsigned long long hits = 0, wedges = 0;
+  int bad = 0, dmax = 0;
+  const int tasks = p.n * p.splits, nwarps = gridDim.x * SM_WARPS;
+  for (int t = blockIdx.x * SM_WARPS + warp; t < tasks; t += nwarps) {
+    const int v = t / p.splits, part = t - v * p.splits;
+    int b;
+    int d = checked_row(p, v, b);
+    if (d < 0) {
+      bad |= TC_DEV_BAD_OFFSETS;
+      continue;
+    }
+    dmax = max(dmax, d);
+    const bool counted = v >= p.row_lo && v < p.row_hi && d >= 2;
+    if (part == 0 && lane < 2) {  // the row's class under the tuned classes and under the plain split
+      const bool plain = lane;
+      const int wm = lane ? TC_PLAIN_WARP_MAX : p.warp_max;
+      int c = TC_CLASS_SKIP;
+      if (counted)
+        c = plain ? (d <= wm ? TC_CLASS_WARP : d <= p.cta_max ? TC_CLASS_CTA : TC_CLASS_HUGE)
+                  : (d <= 4    ? TC_CLASS_G4
+                     : d <= 8  ? TC_CLASS_G8
+                     : d <= 16 ? TC_CLASS_G16
+                     : d <= 32 ? TC_CLASS_G32
+                     : d <= wm ? TC_CLASS_WARP
+                     : d <= p.cta_max ? TC_CLASS_CTA
+                                      : TC_CLASS_HUGE);
+      atomicAdd(&hist[lane][c], 1);
+    }
+    if (part * 32 >= d) continue;
+    if (counted) {
+      for (int i = lane; i < d; i += 32) {
+        const unsigned w = (unsigned)tc_ld_nc(p.adj + b + i);
+        if (w < (unsigned)p.n) atomicOr(words + (w >> 5), 1u << (w & 31u));
+      }
+      __syncwarp();
+    }
+    for (int a0 = part * 32; a0 < d; a0 += 32 * p.splits) {
+      const int i = a0 + lane;
+      int s = 0, dd = 0;
+      if (i < d) {
+        const int u = tc_ld_nc(p.adj + b + i);
+        if ((unsigned)u >= (unsigned)p.n) bad |= p.check_ids ? TC_DEV_BAD_IDS : 0;
+        else if (counted) dd = max(checked_row(p, u, s), 0);
+      }
+      if (!counted) continue;
+      wedges += (unsigned)dd;
+      unsigned h = 0;
+      // four rows at a time, eight lanes each
+      const unsigned have = __ballot_sync(TC_FULL_MASK, dd > 0);
+      for (unsigned rest = have; rest;) {
+        // the grp-th remaining row
+        unsigned mine = rest;
+        for (int k = 0; k < grp; ++k) mine &= mine - 1;
+        const int j = mine ? __ffs(mine) - 1 : 0;
+        const int sj = __shfl_sync(TC_FULL_MASK, s, j);
+        int dj = __shfl_sync(TC_FULL_MASK, dd, j);
+        if (!mine) dj = 0;
+        for (int k = gl; __any_sync(TC_FULL_MASK, k < dj); k += 32) {
+          unsigned w[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) w[r] = k + 8 * r < dj ? (unsigned)tc_ld_nc(p.adj + sj + k + 8 * r) : 0xffffffffu;
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            if (w[r] < (unsigned)p.n) h += words[w[r] >> 5] >> (w[r] & 31u) & 1u;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) rest &= rest - 1;
+      }
+      hits += h;
+    }
+    if (counted) {
+      __syncwarp();
+      for (int i = lane; i < d; i += 32) {
+        const unsigned w = (unsigned)tc_ld_nc(p.adj + b + i);
+        if (w < (unsigned)p.n) words[w >> 5] = 0;
+      }
+      __syncwarp();
+    }
+  }
+  bad = __reduce_or_sync(TC_FULL_MASK, bad);
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    hits += __shfl_down_sync(TC_FULL_MASK, hits, o);
+    wedges += __shfl_down_sync(TC_FULL_MASK, wedges, o);
+  }
+  if (lane == 0) {
+    if (hits) atomicAdd(&s_count, hits);
+    if (wedges) atomicAdd(&s_wedges, wedges);
+    if (bad) atomicOr(&s_bad, bad);
+    atomicMax(&s_dmax, dmax);
+  }
+  __syncthreads();
+  if (threadIdx.x < TC_NUM_CLASSES) {
+    if (hist[0][threadIdx.x]) atomicAdd(&p.acc->class_count[threadIdx.x], hist[0][threadIdx.x]);
+    if (hist[1][threadIdx.x]) atomicAdd(&p.acc->class_count_alt[threadIdx.x], hist[1][threadIdx.x]);
+  }
+  if (threadIdx.x == 0) {
+    if (s_count) atomicAdd(&p.acc->count, s_count);
+    if (s_wedges) atomicAdd(&p.acc->wedges, s_wedges);
+    if (s_bad) atomicOr(&p.acc->status, s_bad);
+    if (s_dmax) atomicMax(&p.acc->max_out_degree, s_dmax);
+  }
+  // the last CTA hands the totals over and clears the accumulators for the next call
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&p.acc->bad_offset_at, 1ull) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  static_assert(sizeof(TcControl) % 8 == 0, "copied by 8-byte words");
+  const unsigned long long *src = reinterpret_cast<const unsigned long long *>(p.acc);
+  for (int i = threadIdx.x; i < (int)(sizeof(TcControl) / 8); i += SM_THREADS) {
+    reinterpret_cast<unsigned long long *>(p.out)[i] = __ldcg(src + i);
+    reinterpret_cast<unsigned long long *>(p.acc)[i] = 0;
+  }
+  __threadfence_system();
+}
+
+}  // namespace
+
+bool small_graph(int64_t n, int64_t m) { return n >= 1 && n <= SMALL_MAX_IDS && m <= SMALL_MAX_ARCS; }
+
+int small_count(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, int64_t row_lo,
+                int64_t row_hi, int check_ids, int warp_max, int cta_max, cudaStream_t st) {
+  if (!c->d_small) {
+    TC_CUDA_TRY(cudaMalloc((void **)&c->d_small, sizeof(TcControl)));
+    TC_CUDA_TRY(cudaMemsetAsync(c->d_small, 0, sizeof(TcControl), st));
+  }
+  SmallArgs a;
+  a.beg = beg;
+  a.adj = adj;
+  a.n = (int)n;
+  a.m = (int)m;
+  a.row_lo = (int)row_lo;
+  a.row_hi = (int)row_hi;
+  a.check_ids = check_ids;
+  a.warp_max = warp_max;
+  a.cta_max = cta_max;
+  // rows of few batches: a warp each; dense graphs: several warps share a row's batches
+  a.splits = (int)std::min<int64_t>(8, std::max<int64_t>(1, m / (16 * n)));
+  a.words = (int)((n + 31) / 32);
+  a.acc = c->d_small;
+  a.out = c->h_ctl;
+  const int64_t tasks = n * a.splits;
+  const size_t smem = sizeof(unsigned) * (size_t)a.words * SM_WARPS;
+  TC_CUDA_TRY(cudaFuncSetAttribute(small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(SMALL_MAX_IDS / 8 * SM_WARPS)));
+  const int per_sm = (int)std::min<size_t>(6, (size_t)220 * 1024 / (smem + 1536));  // resident CTAs
+  const int blocks = (int)std::min<int64_t>((tasks + SM_WARPS - 1) / SM_WARPS, (int64_t)c->num_sms * per_sm);
+  small_kernel<<<blocks, SM_THREADS, smem, st>>>(a);
+  note_launch();
+  TC_CUDA_TRY(cudaGetLastError());
+  return TRUST_TC_OK;
+}
+
+}  // namespace tc
