@@ -22,6 +22,7 @@
 #include "tc_count.h"
 #include "tc_internal.h"
 #include "tc_model.h"
+#include "tc_short.h"
 #include "tc_small.h"
 
 namespace tc {
@@ -196,6 +197,10 @@ constexpr double TC_LEARNED_MIN_LONG_FRAC = 0.15;
 // graphs (longest rows 18 to 29 entries: 0.09 / 0.20, 0.11 / 0.14, 0.09 / 0.12) the tuned classes win.
 constexpr int64_t TC_SMALL_SKEWED_ARCS = (int64_t)1 << 21;
 constexpr int TC_SMALL_SKEWED_MIN_ROW = 64;
+
+// Graphs of at least this many rows, none longer than 8, are counted by the row-order kernel: mesh
+// 300 x 300 89 -> 64 us, Erdos-Renyi 100,000 / 250,000 arcs 88 -> 63 us; smaller ones take one launch.
+constexpr int64_t TC_SHORT_MIN_ROWS = 1 << 16;
 
 // Make the cost model in use resident on the device: the caller's (opts.model) or the library's
 // default.  Sets *d_model to null when neither is available (no decisions from a model).
@@ -525,7 +530,13 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     rc = bits_launch(c, bits, g.adjA, ctl, st);
     if (rc) return rc;
   }
-  rc = launch_count(same, a, blocks, cfg.threads, smem, st);
+  // a large graph of short rows only: the row-order kernel
+  const bool short_rows = same && !g.rowmap && g.min_deg == 2 && o.schedule != TRUST_TC_SCHED_PLAIN && !o.record_cycles &&
+                          !split && g.rows >= TC_SHORT_MIN_ROWS && h.max_out_degree <= SHORT_ROW_MAX;
+  if (short_rows)
+    rc = launch_short_rows(g.begA, g.adjA, g.rows, g.mA, row_lo, row_hi < 0 ? g.rows : row_hi, ctl, c->num_sms, st);
+  else
+    rc = launch_count(same, a, blocks, cfg.threads, smem, st);
   if (rc) return rc;
   TC_CUDA_TRY(cudaEventRecord(c->ev[3], st));
   TC_CUDA_TRY(cudaMemcpyAsync(c->h_ctl, ctl, sizeof(TcControl), cudaMemcpyDeviceToHost, st));
