@@ -1,0 +1,81 @@
+"""The batch counting kernel (tc_batch_count.cu) where its row sets change: graphs around the sizes
+whose ids fit a warp's bitmap or half of it, rows of every class up to spill tables, dense graphs,
+and buffers refilled after the batch was made."""
+import numpy as np
+import pytest
+
+import trust_gb300 as T
+from trust_gb300 import batch as B
+from oracle import oracle as O
+from tests import graphs
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _er(rng, n, deg):
+    return O.build_csr(rng.integers(0, n, size=(n * deg // 2, 2)).astype(np.int32), n)
+
+
+def _hub(rng, n, longest):
+    """Row 0 of `longest` entries, every other row up to 40: not oriented, sorted, no duplicates."""
+    rows = [np.sort(rng.choice(n, size=longest, replace=False))]
+    rows += [np.unique(rng.integers(0, n, size=rng.integers(0, 41))) for _ in range(n - 1)]
+    beg = np.concatenate([[0], np.cumsum([r.size for r in rows])]).astype(np.int64)
+    return beg, np.concatenate(rows).astype(np.int32)
+
+
+def _union(csrs):
+    vb = np.concatenate([[0], np.cumsum([b.size - 1 for b, _ in csrs])]).astype(np.int64)
+    eb = np.concatenate([[0], np.cumsum([a.size for _, a in csrs])]).astype(np.int64)
+    beg = np.concatenate([b[:-1] + eb[g] for g, (b, _) in enumerate(csrs)] + [eb[-1:]])
+    adj = np.concatenate([a + np.int32(vb[g]) for g, (_, a) in enumerate(csrs)])
+    return torch.from_numpy(beg).cuda(), torch.from_numpy(adj.astype(np.int32)).cuda(), vb
+
+
+def _check(csrs, settings=((256, 128, 8),)):
+    beg, adj, vb = _union(csrs)
+    expect = np.array([O.count_forward(b, a, threads=8) for b, a in csrs], dtype=np.uint64)
+    wedges = sum(O.wedges(b, a) for b, a in csrs)
+    with T.Context() as ctx:
+        bt = B.Batch(beg, adj, vb, ctx=ctx)
+        for threads, warp_max, chunk in settings:
+            for s in range(4):
+                bt.set_class(s, threads, warp_max, chunk)
+            for _ in range(2):
+                counts, r = bt.run()
+                assert np.array_equal(counts, expect)
+                assert r.triangles == int(expect.sum()) and r.wedges == wedges
+        bt.close()
+
+
+@pytest.mark.parametrize("n", [25_088, 25_089, 50_176, 50_177, 51_200, 51_201, 70_000])
+def test_bitmap_bounds(n):
+    rng = np.random.default_rng(n)
+    _check([_er(rng, n, 24), _er(rng, 300, 40), _er(rng, n, 64), _er(rng, 7, 3)])
+
+
+@pytest.mark.parametrize("settings", [((256, 128, 8), (1024, 64, 4)), ((64, 32, 1), (512, 1024, 16))])
+def test_every_class(settings):
+    rng = np.random.default_rng(11)
+    cs = [O.build_csr(graphs.complete(k)[0], k) for k in (3, 5, 9, 17, 33, 34, 130, 300)]
+    cs += [_hub(rng, 6000, 5000), _hub(rng, 90_000, 3000), _er(rng, 900, 100)]
+    _check(cs, settings)
+
+
+def test_refilled_buffers():
+    """A run counts what the buffers hold: other graphs of the same sizes, and an arc that leaves its
+    graph (out of its bitmap's range) is looked up as any other entry."""
+    rng = np.random.default_rng(5)
+    cs = [_er(rng, 400, 30), _er(rng, 400, 30)]
+    beg, adj, vb = _union(cs)
+    with T.Context() as ctx:
+        bt = B.Batch(beg, adj, vb, ctx=ctx)
+        a = adj.cpu().numpy().copy()
+        b = beg.cpu().numpy()
+        v = int(np.argmax(np.diff(b)[:400]))  # a long row of graph 0: its last two entries leave the graph
+        a[b[v + 1] - 2:b[v + 1]] = [int(vb[1]) + 3, int(vb[1]) + 4]
+        adj.copy_(torch.from_numpy(a))
+        counts, r = bt.run()
+        assert r.triangles == int(counts.sum()) == O.count_forward(b, a)
+        bt.close()

@@ -8,7 +8,7 @@
 // class of its graph, degree class) with each size class's own warp-class bound, list offsets
 // computed on the device (degree class major, so every degree class is one list over all size
 // classes), one persistent counting kernel over all of them, and the readback of the per-graph
-// counts.  Hits are attributed to graphs inside the counting kernel (CountArgs graph_of /
+// counts.  Hits are attributed to graphs inside the counting kernel (tc_batch_count.cu: graph_of /
 // graph_counts).  One launch instead of one per size class: measured on GB300 for the 4096-graph
 // workload, 14.6 ms for the union in one launch against 16.8 ms for four autotuned per-class
 // launches (the classes' kernels ran one after another, each draining to its own tail).  The
@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "tc_batch_count.h"
 #include "tc_count.h"
 #include "tc_internal.h"
 
@@ -28,6 +29,9 @@ namespace {
 
 // size classes by vertex count: [0, 512), [512, 4096), [4096, 32768), [32768, ...)
 constexpr int64_t SC_LIMIT[TC_BATCH_CLASSES - 1] = {512, 4096, 32768};
+// Bitmap words per warp: graphs of up to 50,176 vertices, and still four CTAs of eight warps per SM
+// (4096 graphs of up to 50,000, ms per run: 512 words 17.1, 1024 15.4, 1568 13.9).
+constexpr int BITMAP_WORDS = 1568;
 constexpr int CTA_MAX = 4096;  // CTA-class bound of every size class (hub rows above it spill)
 
 int size_class_of(int64_t nv) {
@@ -83,10 +87,11 @@ struct trust_tc_batch {
   const int32_t *adj = nullptr;
   int64_t n = 0, m = 0, G = 0;
   int64_t graphs[TC_BATCH_CLASSES] = {}, vertices[TC_BATCH_CLASSES] = {};
+  int64_t max_vertices[TC_BATCH_CLASSES] = {};  // of one graph
   int maxdeg[TC_BATCH_CLASSES] = {};
   trust_tc_batch_class cfg[TC_BATCH_CLASSES];
   // the resolved counting launch (one for every size class)
-  int threads = 256, chunk = 8, blocks = 0, warp_slots = 0, long_cap = 0;
+  int threads = 256, chunk = 8, blocks = 0, warp_words = 0;
   size_t smem = 0;
   int64_t *d_vbeg = nullptr;
   int *d_graph_of = nullptr;
@@ -97,8 +102,6 @@ struct trust_tc_batch {
   int *d_lists = nullptr;
   int *d_huge = nullptr;
   int huge_log2 = 0, huge_blocks = 0;
-  int2 *d_long = nullptr;
-  size_t long_bytes = 0;
   cudaStream_t st = nullptr;
   cudaGraphExec_t exec = nullptr;
   uint64_t kernels_per_run = 0;
@@ -119,7 +122,6 @@ void batch_release(trust_tc_batch *b) {
   cudaFreeHost(b->h_ctl);
   cudaFree(b->d_lists);
   cudaFree(b->d_huge);
-  cudaFree(b->d_long);
   for (auto e : b->ev)
     if (e) cudaEventDestroy(e);
   if (b->st) cudaStreamDestroy(b->st);
@@ -157,26 +159,25 @@ int batch_prepare(trust_tc_batch *b) {
       dcta = std::max(dcta, std::min(b->maxdeg[s], CTA_MAX));
     }
   }
-  b->warp_slots = std::max(slots, 128);
-  size_t sm = (size_t)4 * b->warp_slots * warps;
+  // the bitmap of a graph's ids where that takes at most BITMAP_WORDS words per warp, and the 32 keys
+  // of the group classes
+  int64_t ids = 0;
+  for (int s = 0; s < TC_BATCH_CLASSES; ++s)
+    if (b->graphs[s] && b->maxdeg[s] > 8) ids = std::max(ids, b->max_vertices[s]);
+  b->warp_words = std::max(std::max(slots, 128), (int)std::min<int64_t>((ids + 127) / 128 * 4, BITMAP_WORDS) + 32);
+  size_t sm = (size_t)4 * b->warp_words * warps;
+  if (sm > (size_t)b->ctx->max_smem_optin) {  // many warps: what the hash tables need
+    b->warp_words = std::max(slots, 128);
+    sm = (size_t)4 * b->warp_words * warps;
+  }
   if (cta) sm = std::max(sm, (size_t)4 << std::max(ceil_log2(2 * (int64_t)dcta), 6));
   if (sm > (size_t)b->ctx->max_smem_optin) return TRUST_TC_E_ARG;
   b->smem = sm;
   int per_sm = 0;
-  int rc = count_kernel_occupancy(true, b->threads, sm, &per_sm);
+  int rc = batch_count_occupancy(b->threads, sm, &per_sm);
   if (rc) return rc;
   if (per_sm < 1) return TRUST_TC_E_ARG;
   b->blocks = num_sms * per_sm;
-  b->long_cap = dcta;
-  if ((rc = set_count_kernel_carveout(true, b->threads, sm, per_sm))) return rc;
-  const size_t long_need = sizeof(int2) * (size_t)b->long_cap * (size_t)b->blocks;
-  if (long_need > b->long_bytes) {
-    cudaFree(b->d_long);
-    b->d_long = nullptr;
-    b->long_bytes = 0;
-    TC_CUDA_TRY(cudaMalloc((void **)&b->d_long, long_need));
-    b->long_bytes = long_need;
-  }
   return TRUST_TC_OK;
 }
 
@@ -199,24 +200,22 @@ int batch_enqueue(trust_tc_batch *b, cudaStream_t st, bool timed) {
   if ((rc = launch_batch_classify(1, b->beg, b->n, b->d_graph_of, b->d_graph_sc, th, b->d_ctl, b->d_lists, num_sms,
                                   st)))
     return rc;
-  CountArgs a{};
-  a.begA = a.begB = a.begC = b->beg;
-  a.adjA = a.adjB = a.adjC = b->adj;
-  a.rows = b->n;
+  BatchCountArgs a{};
+  a.beg = b->beg;
+  a.adj = b->adj;
   a.lists = b->d_lists;
   a.ctl = b->d_ctl + TC_BATCH_CLASSES;  // the combined lists of every size class
+  a.graph_of = b->d_graph_of;
+  a.graph_vbeg = b->d_vbeg;
+  a.graph_counts = b->d_counts;
   a.huge_tables = b->d_huge;
   a.huge_log2 = b->huge_log2;
   a.huge_blocks = std::min(b->huge_blocks, b->blocks);
-  a.warp_slots = b->warp_slots;
+  a.warp_words = b->warp_words;
+  a.table_bytes = (int)b->smem;
   a.chunk = b->chunk;
-  a.long_rows = b->d_long;
-  a.long_cap = b->long_cap;
-  a.graph_of = b->d_graph_of;
-  a.graph_counts = b->d_counts;
-  a.dev_off = 1;
   if (timed) TC_CUDA_TRY(cudaEventRecord(b->ev[2], st));
-  if ((rc = launch_count(true, a, b->blocks, b->threads, b->smem, st))) return rc;
+  if ((rc = launch_batch_count(a, b->blocks, b->threads, st))) return rc;
   if (timed) TC_CUDA_TRY(cudaEventRecord(b->ev[3], st));
   TC_CUDA_TRY(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(TcControl) * NCTL, cudaMemcpyDeviceToHost, st));
   TC_CUDA_TRY(cudaMemcpyAsync(b->h_counts, b->d_counts, sizeof(unsigned long long) * (size_t)b->G,
@@ -289,6 +288,7 @@ int trust_tc_batch_create(trust_tc_ctx *ctx, const int64_t *d_begin, const int32
     sc[(size_t)g] = (unsigned char)size_class_of(nv);
     b->graphs[sc[(size_t)g]] += 1;
     b->vertices[sc[(size_t)g]] += nv;
+    b->max_vertices[sc[(size_t)g]] = std::max(b->max_vertices[sc[(size_t)g]], nv);
   }
   for (auto &c : b->cfg) c = trust_tc_batch_class{256, 128, 8};
   auto fail = [&](int rc) {

@@ -771,39 +771,8 @@ __device__ __forceinline__ void row_of(const int64_t *__restrict__ beg, int v, i
   d = (int)(hi - lo);
 }
 
-// The list of class c (offsets from the host, or computed on the device for batches).
-__device__ __forceinline__ const int *class_list(const CountArgs &p, int c) {
-  return p.lists + (p.dev_off ? p.ctl->class_off[c] : p.off.off[c]);
-}
-template <bool BATCH>
-__device__ __forceinline__ const int *class_list_t(const CountArgs &p, int c) {
-  if constexpr (BATCH) return p.lists + p.ctl->class_off[c];
-  else return p.lists + p.off.off[c];
-}
-
-// Per-graph attribution of a batch.  Every lane keeps the hits of the graph its warp is
-// currently working on; when the warp moves to another graph the warp's sum goes to that graph's
-// counter with one atomic.  Calls are warp-uniform (same g in every lane).
-struct BatchAcc {
-  int cur;
-  unsigned long long h;
-};
-
-__device__ __forceinline__ void batch_flush(const CountArgs &p, BatchAcc &a) {
-  unsigned long long s = a.h;
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) s += __shfl_xor_sync(TC_FULL_MASK, s, off);
-  if ((threadIdx.x & 31) == 0 && a.cur >= 0 && s) atomicAdd(p.graph_counts + a.cur, s);
-  a.h = 0;
-}
-
-__device__ __forceinline__ void batch_take(const CountArgs &p, BatchAcc &a, int g, unsigned long long delta) {
-  if (g != a.cur) {
-    batch_flush(p, a);
-    a.cur = g;
-  }
-  a.h += delta;
-}
+// The list of class c.
+__device__ __forceinline__ const int *class_list(const CountArgs &p, int c) { return p.lists + p.off.off[c]; }
 
 // One vertex handled by a whole CTA.  `tab` is shared (CTA class) or global (huge class).
 // Pass 1: warps claim 32-arc batches from a shared counter; short rows are flattened and probed
@@ -963,17 +932,15 @@ struct GroupStage {
 // Drain one group class.  Each warp claims `chunk` steps of 32/G vertices.  Loads run three
 // steps ahead: while step t is probed, step t+1's target rows, step t+2's row elements and
 // step t+3's row bounds are in flight (the reference walks this chain serially per vertex).
-// BATCH: the batch instantiation (per-graph attribution, device list offsets); the single-graph
-// kernel carries none of its state.
-template <int G, bool SAME, bool REC, bool BATCH>
+template <int G, bool SAME, bool REC>
 __device__ void drain_group_class(const CountArgs &p, int c, int *warp_tab, unsigned long long &hits,
-                                  unsigned long long &wedges, BatchAcc &acc) {
+                                  unsigned long long &wedges) {
   constexpr int GPW = 32 / G;
   const int lane = threadIdx.x & 31;
   const int g = lane / G;
   const int glane = lane & (G - 1);
   const int n_items = p.ctl->class_count[c];
-  const int *list = class_list_t<BATCH>(p, c);
+  const int *list = class_list(p, c);
   const int claim = p.chunk * GPW;
   // stage loaders
   auto ld_v = [&](int item, int t1) { return item < t1 ? list[item] : -1; };
@@ -1019,22 +986,7 @@ __device__ void drain_group_class(const CountArgs &p, int c, int *warp_tab, unsi
       ld_elem(s2);
       ld_row(s3);
       const long long t_start = REC ? clock64() : 0;
-      if constexpr (!BATCH) {
-        group_vertex<G, SAME>(p, s0.uA, s0.s, s0.dd, warp_tab, hits, wedges);
-      } else {
-        // a batch: one pass per graph present in this step (almost always one), the other
-        // groups' vertices masked out, so every hit of a pass belongs to that pass's graph
-        const int gid = s0.v >= 0 ? p.graph_of[s0.v] : -1;
-        unsigned pending = __ballot_sync(TC_FULL_MASK, gid >= 0);
-        while (pending) {
-          const int gx = __shfl_sync(TC_FULL_MASK, gid, __ffs(pending) - 1);
-          const bool mine = gid == gx;
-          const unsigned long long h0 = hits;
-          group_vertex<G, SAME>(p, mine ? s0.uA : -1, s0.s, mine ? s0.dd : 0, warp_tab, hits, wedges);
-          batch_take(p, acc, gx, hits - h0);
-          pending &= ~__ballot_sync(TC_FULL_MASK, mine);
-        }
-      }
+      group_vertex<G, SAME>(p, s0.uA, s0.s, s0.dd, warp_tab, hits, wedges);
       if (REC) {
         // the step's cycles, shared among its vertices in proportion to their wedges
         const long long dt = clock64() - t_start;
@@ -1058,7 +1010,7 @@ __device__ void drain_group_class(const CountArgs &p, int c, int *warp_tab, unsi
 // with at least TC_MIN_CTAS_256 CTAs resident per SM (the default shape).
 constexpr int TC_MIN_CTAS_256 = 5;
 
-template <bool SAME, bool REC, int MAXT, int MINB, bool BATCH>
+template <bool SAME, bool REC, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) count_kernel(CountArgs p) {
   extern __shared__ int smem[];
   __shared__ BlockShared bs;
@@ -1066,14 +1018,13 @@ __global__ void __launch_bounds__(MAXT, MINB) count_kernel(CountArgs p) {
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) bs.count = bs.wedges = 0;
   unsigned long long hits = 0, wedges = 0;
-  BatchAcc acc{-1, 0};
 
   // Phase A: CTA-granularity vertices, largest class first.
   for (int c = TC_CLASS_HUGE; c >= TC_CLASS_CTA; --c) {
     const int n_items = p.ctl->class_count[c];
     if (n_items == 0 || (c == TC_CLASS_HUGE && p.table_min > 0)) continue;
     if (c == TC_CLASS_HUGE && (int)blockIdx.x >= p.huge_blocks) continue;
-    const int *list = class_list_t<BATCH>(p, c);
+    const int *list = class_list(p, c);
     int *tab = (c == TC_CLASS_HUGE) ? p.huge_tables + (size_t)blockIdx.x * ((size_t)1 << p.huge_log2)
                                     : smem;
     for (;;) {
@@ -1094,10 +1045,8 @@ __global__ void __launch_bounds__(MAXT, MINB) count_kernel(CountArgs p) {
         if (d > p.table_min) continue;
       }
       const long long t_start = REC ? clock64() : 0;
-      const unsigned long long h0 = hits;
       cta_vertex<SAME>(p, v, tab, c == TC_CLASS_CTA, bs, hits, wedges);
       if (REC && threadIdx.x == 0) p.cycles[v] = (unsigned long long)(clock64() - t_start);
-      if constexpr (BATCH) batch_take(p, acc, p.graph_of[v], hits - h0);
     }
   }
   __syncthreads();
@@ -1107,7 +1056,7 @@ __global__ void __launch_bounds__(MAXT, MINB) count_kernel(CountArgs p) {
   {
     const int c = TC_CLASS_WARP;
     const int n_items = p.ctl->class_count[c];
-    const int *list = class_list_t<BATCH>(p, c);
+    const int *list = class_list(p, c);
     for (;;) {
       int t0 = 0;
       // warp-class vertices are large: claim them one at a time unless the chunk is very coarse
@@ -1124,18 +1073,15 @@ __global__ void __launch_bounds__(MAXT, MINB) count_kernel(CountArgs p) {
           if (d > p.table_min) continue;
         }
         const long long t_start = REC ? clock64() : 0;
-        const unsigned long long h0 = hits;
         warp_vertex<SAME>(p, v, warp_tab, hits, wedges);
         if (REC && lane == 0) p.cycles[v] = (unsigned long long)(clock64() - t_start);
-        if constexpr (BATCH) batch_take(p, acc, p.graph_of[v], hits - h0);
-      }
+        }
     }
   }
-  drain_group_class<32, SAME, REC, BATCH>(p, TC_CLASS_G32, warp_tab, hits, wedges, acc);
-  drain_group_class<16, SAME, REC, BATCH>(p, TC_CLASS_G16, warp_tab, hits, wedges, acc);
-  drain_group_class<8, SAME, REC, BATCH>(p, TC_CLASS_G8, warp_tab, hits, wedges, acc);
-  drain_group_class<4, SAME, REC, BATCH>(p, TC_CLASS_G4, warp_tab, hits, wedges, acc);
-  if constexpr (BATCH) batch_flush(p, acc);
+  drain_group_class<32, SAME, REC>(p, TC_CLASS_G32, warp_tab, hits, wedges);
+  drain_group_class<16, SAME, REC>(p, TC_CLASS_G16, warp_tab, hits, wedges);
+  drain_group_class<8, SAME, REC>(p, TC_CLASS_G8, warp_tab, hits, wedges);
+  drain_group_class<4, SAME, REC>(p, TC_CLASS_G4, warp_tab, hits, wedges);
 
   // Reduction: warp shuffle -> shared u64 -> one global u64 atomic per CTA
   // (the reference does per-thread shared atomics, Without-graph-partition/TC.cu:586-599).
@@ -1504,9 +1450,8 @@ int launch_classify(int pass, const int64_t *begA, const int64_t *begB, int64_t 
 template <bool SAME, int MAXT, int MINB>
 static cudaError_t occupancy_of(int threads, size_t smem_bytes, int *blocks_per_sm) {
   cudaError_t e = cudaSuccess;
-  const void *fns[3] = {(const void *)count_kernel<SAME, false, MAXT, MINB, false>,
-                        (const void *)count_kernel<SAME, true, MAXT, MINB, false>,
-                        (const void *)count_kernel<SAME, false, MAXT, MINB, SAME>};
+  const void *fns[2] = {(const void *)count_kernel<SAME, false, MAXT, MINB>,
+                        (const void *)count_kernel<SAME, true, MAXT, MINB>};
   for (const void *fn : fns)
     if (e == cudaSuccess) e = set_attr(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes, true);
   if (e != cudaSuccess) return e;
@@ -1525,7 +1470,7 @@ static cudaError_t occupancy_of(int threads, size_t smem_bytes, int *blocks_per_
   for (const void *fn : fns)
     if (e == cudaSuccess) e = set_attr(fn, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
   if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, count_kernel<SAME, false, MAXT, MINB, false>, threads,
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, count_kernel<SAME, false, MAXT, MINB>, threads,
                                                       smem_bytes);
   if (e == cudaSuccess) {
     AttrCache &c = attr_cache();
@@ -1550,9 +1495,8 @@ int count_kernel_occupancy(bool same, int threads, size_t smem_bytes, int *block
 template <bool SAME, int MAXT, int MINB>
 static cudaError_t carveout_of(int pct) {
   cudaError_t e = cudaSuccess;
-  for (const void *fn : {(const void *)count_kernel<SAME, false, MAXT, MINB, false>,
-                         (const void *)count_kernel<SAME, true, MAXT, MINB, false>,
-                         (const void *)count_kernel<SAME, false, MAXT, MINB, SAME>})
+  for (const void *fn :
+       {(const void *)count_kernel<SAME, false, MAXT, MINB>, (const void *)count_kernel<SAME, true, MAXT, MINB>})
     if (e == cudaSuccess) e = set_attr(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
   return e;
 }
@@ -1573,12 +1517,10 @@ int set_count_kernel_carveout(bool same, int threads, size_t smem_bytes, int per
 
 template <bool SAME, int MAXT, int MINB>
 static void launch_one(const CountArgs &a, int blocks, int threads, size_t smem_bytes, cudaStream_t st) {
-  if (SAME && a.graph_of)  // batches: one graph CSR, no cycle recording
-    count_kernel<SAME, false, MAXT, MINB, SAME><<<blocks, threads, smem_bytes, st>>>(a);
-  else if (a.cycles)
-    count_kernel<SAME, true, MAXT, MINB, false><<<blocks, threads, smem_bytes, st>>>(a);
+  if (a.cycles)
+    count_kernel<SAME, true, MAXT, MINB><<<blocks, threads, smem_bytes, st>>>(a);
   else
-    count_kernel<SAME, false, MAXT, MINB, false><<<blocks, threads, smem_bytes, st>>>(a);
+    count_kernel<SAME, false, MAXT, MINB><<<blocks, threads, smem_bytes, st>>>(a);
   TC_NOTE_LAUNCH();
 }
 

@@ -33,11 +33,6 @@ struct CountArgs {
   const int *rowmap;  // optional: table row (A) of each work row (B); null = the same index
   int2 *long_rows;    // optional: per-CTA lists of deferred long neighbour rows (row start, length)
   int long_cap;       // entries per CTA in long_rows (>= the largest CTA-class out-degree)
-  // batches (the disjoint union of many graphs): graph of every row, per-graph counts (both null
-  // otherwise), and list offsets read from ctl->class_off on the device instead of `off`
-  const int *graph_of;
-  unsigned long long *graph_counts;
-  int dev_off;
   // huge rows up to this out-degree are counted by hub_kernel in shared memory (0: none)
   int hub_max_degree;
   // failure-detection test: hub_kernel arms its copy barrier without issuing the copy and waits
