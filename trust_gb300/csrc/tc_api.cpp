@@ -101,6 +101,8 @@ void ctx_release(trust_tc_ctx *c) {
   cudaFree(c->d_split_wsum);
   cudaFree(c->d_split_plans);
   cudaFree(c->d_sched_long);
+  cudaFree(c->d_split_place);
+  cudaFree(c->d_deg);
   cudaFree(c->d_split_pairs);
   cudaFree(c->d_split_beg);
   cudaFree(c->d_split_cbase);

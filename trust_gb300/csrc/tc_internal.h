@@ -19,7 +19,7 @@ struct trust_tc_ctx {
   size_t huge_cap = 0;
   int2 *d_long = nullptr;  // per-CTA deferred long-row lists of the CTA class
   size_t long_cap = 0;
-  unsigned *d_split_cnt = nullptr;  // direction split: in-degree counts / scatter cursors
+  unsigned *d_split_cnt = nullptr;  // direction split: in-list lengths
   size_t split_cnt_cap = 0;
   unsigned char *d_dec = nullptr;  // learned schedule: class decision of every row longer than 32
   size_t dec_cap = 0;
@@ -39,6 +39,10 @@ struct trust_tc_ctx {
   unsigned long long *h_plans = nullptr;        // pinned host copy of d_split_plans
   int2 *d_split_pairs = nullptr;  // scheduling pass: the arcs the split would move, (target, source)
   size_t split_pairs_cap = 0;
+  unsigned *d_split_place = nullptr;  // and each one's place in its target's in-list
+  size_t split_place_cap = 0;
+  int *d_deg = nullptr;  // scheduling pass: out-degrees
+  size_t deg_cap = 0;
   int *d_sched_long = nullptr;  // scheduling pass: the rows it walks a warp each
   size_t sched_long_cap = 0;
   int64_t *d_split_beg = nullptr;  // in-list offsets of the arcs sent to the second pass
@@ -134,8 +138,8 @@ struct SchedPlan {
   bool overflow;                    // the pair arrays ran out (never expected): no split
 };
 // Only source rows in [row_lo, row_hi) are walked (their arcs planned and moved).  An arc (v,u) is
-// moved to u's side when d(u) > max(d(v), table_min); with table_min > 0 the work sum of a row
-// longer than table_min also holds the probes of the arcs it keeps.
+// moved to u's side when d(u) > max(d(v), table_min).  Work sums: the probes of the arcs moved to a
+// row; with table_min > 0 instead those of the arcs that a row longer than table_min keeps.
 int split_plan(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, cudaStream_t st,
                const float *d_model, int warp_max, int cta_max, float promote_log2, int cta_warps, TcControl *ctl,
                int64_t row_lo, int64_t row_hi, int table_min);
@@ -149,6 +153,8 @@ int vertex_features(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int
 // probes each, so the table rebuild stays a small fraction of a row's work
 constexpr int TC_SPLIT_WORK_PER_ENTRY = 256;
 constexpr int TC_SPLIT_MIN_WORK = 131072;
+// The moved arcs' sources at their places of c->d_split_adj, u's in-list starting at off[u].
+int split_fill_u32(trust_tc_ctx *c, int64_t m, const unsigned *off, cudaStream_t st);
 struct SplitRows {
   const int64_t *beg;
   const int32_t *adj;
