@@ -139,3 +139,17 @@ def test_partitioned_folder_direction_split(tmp_path):
     T.partition_folder(str(tmp_path), b, a, 3)
     r = T.count_partitioned(str(tmp_path), 3, direction_split=1)
     assert r.triangles == expect and r.direction_split >= 1
+
+
+@pytest.mark.parametrize("p", [1, 2, 3, 7])
+@pytest.mark.parametrize("room", [0, 1])
+def test_device_tiles_at_the_budget(p, room):
+    """A budget that just holds all tiles keeps them on the device, one byte less streams them: the
+    same result either way (7 parts: tiles of very different alignment and size)."""
+    beg, adj, expect = _sorted_csr("rmat12")
+    n, m = beg.numel() - 1, adj.numel()
+    rows = sum((n - i + p - 1) // p + 1 for i in range(p)) * p
+    r = T.count_tiles(beg, adj, p, budget_bytes=8 * rows + 4 * m - 1 + room)
+    whole = T.count_tiles(beg, adj, p)
+    assert r.triangles == whole.triangles == expect
+    assert (r.wedges, r.edges, r.vertices, r.class_sizes) == (whole.wedges, whole.edges, whole.vertices, whole.class_sizes)

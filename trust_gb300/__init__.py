@@ -199,8 +199,9 @@ def autotune(beg, adj, ctx: Context, repeats: int = 3, schedule=SCHED_LEARNED,
 
 def count_tiles(beg, adj, parts: int, budget_bytes: int = 0, threads=0, blocks=0, chunk=0,
                 schedule=SCHED_LEARNED, direction_split: int = -1) -> CountResult:
-    """The n x n tile loop over a device CSR (torch CUDA tensors): GPU partition into pinned host
-    tiles, then the (i,j,k) jobs with tiles streamed into a device cache of `budget_bytes`.
+    """The n x n tile loop over a device CSR (torch CUDA tensors): GPU partition into tiles,
+    then the (i,j,k) jobs; tiles that do not all fit a device cache of `budget_bytes` are streamed
+    into it from pinned host memory.
     `direction_split`: -1 the schedule decides per job, 0 never, 1 every job whose tiles allow it
     (`CountResult.direction_split` = the jobs that ran it)."""
     o = _opts(threads, blocks, chunk, DEVICE, schedule=schedule)

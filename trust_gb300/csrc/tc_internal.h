@@ -121,14 +121,16 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
 size_t scan_u32_scratch(int64_t n);
 int scan_exclusive_u32(const unsigned *in, unsigned *out, int64_t n, unsigned *scratch, cudaStream_t st);
 int scan_exclusive_i64(const int64_t *in, int64_t *out, int64_t n, cudaStream_t st, int64_t *total);
-// The n x n hash partition of a device CSR into p*p tiles (tile i*p+j) in pinned host memory
-// (free each beg / adj with cudaFreeHost); p <= 32.
-struct PinnedTile {
+// The n x n hash partition of a device CSR into p*p tiles (tile i*p+j), p <= 32: all tiles in two device
+// blocks, which the caller frees with cudaFree.  Complete when it returns.
+struct Tile {
   int64_t *beg;
-  int32_t *adj;
+  int32_t *adj;  // 256-byte aligned
   int64_t rows, m;
+  size_t bytes() const { return sizeof(int64_t) * (size_t)(rows + 1) + sizeof(int32_t) * (size_t)(m > 0 ? m : 1); }
 };
-int partition_device_to_host(const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, int p, PinnedTile *tiles);
+int partition_device(const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, int p, Tile *tiles, int64_t **d_beg,
+                     int32_t **d_adj);
 constexpr int TC_PLAN_WORDS = 8;  // words of the scheduling pass's totals
 struct SchedPlan {
   unsigned long long w_all, w_min;  // probes without / with the direction split

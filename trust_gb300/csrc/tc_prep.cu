@@ -725,16 +725,16 @@ __global__ void part_fill_kernel(const int64_t *__restrict__ beg, const int32_t 
 
 namespace tc {
 
-int partition_device_to_host(const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, int p, PinnedTile *tiles) {
+int partition_device(const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, int p, Tile *tiles, int64_t **d_beg,
+                     int32_t **d_adj) {
   if (n < 1 || m < 0 || p < 1 || p > 32) return TRUST_TC_E_ARG;
   cudaStream_t st = 0;
   const int64_t stride = (n + p - 1) / p + 1;  // rows of part 0, plus the end offset
   const size_t T = (size_t)p * p;
   int64_t *cnt = nullptr, *tbase = nullptr;
   int32_t *out = nullptr;
-  for (size_t t = 0; t < T; ++t) tiles[t] = PinnedTile{};
   TC_CUDA_TRY(cudaMalloc((void **)&cnt, sizeof(int64_t) * T * (size_t)stride));
-  auto done = [&](int rc) {
+  auto fail = [&](int rc) {
     cudaFree(cnt);
     cudaFree(tbase);
     cudaFree(out);
@@ -742,45 +742,38 @@ int partition_device_to_host(const int64_t *beg, const int32_t *adj, int64_t n, 
   };
   auto cu = [&](cudaError_t e) { return e == cudaSuccess ? TRUST_TC_OK : cuda_status(e); };
   int rc = cu(cudaMemsetAsync(cnt, 0, sizeof(int64_t) * T * (size_t)stride, st));
-  if (rc) return done(rc);
+  if (rc) return fail(rc);
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n * 32 + 255) / 256, 152 * 64));
   part_count_kernel<<<blocks, 256, 0, st>>>(beg, adj, n, p, stride, cnt);
   TC_NOTE_LAUNCH();
-  if ((rc = cu(cudaGetLastError()))) return done(rc);
+  if ((rc = cu(cudaGetLastError()))) return fail(rc);
   std::vector<int64_t> hbase(T + 1, 0);
+  int64_t all = 0;
   for (size_t t = 0; t < T; ++t) {
     const int i = (int)(t / p);
     const int64_t rows = n > i ? (n - i + p - 1) / p : 0;
     int64_t total = 0;
-    if ((rc = scan_exclusive_i64(cnt + t * stride, cnt + t * stride, rows + 1, st, &total))) return done(rc);
+    if ((rc = scan_exclusive_i64(cnt + t * stride, cnt + t * stride, rows + 1, st, &total))) return fail(rc);
     tiles[t].rows = rows;
     tiles[t].m = total;
-    hbase[t + 1] = hbase[t] + total;
+    all += total;
+    hbase[t + 1] = (hbase[t] + total + 63) & ~(int64_t)63;
   }
-  if (hbase[T] != m) return done(TRUST_TC_E_DEVICE);
-  if ((rc = cu(cudaMalloc((void **)&tbase, sizeof(int64_t) * (T + 1))))) return done(rc);
-  if ((rc = cu(cudaMalloc((void **)&out, sizeof(int32_t) * (size_t)std::max<int64_t>(m, 1))))) return done(rc);
-  if ((rc = cu(cudaMemcpy(tbase, hbase.data(), sizeof(int64_t) * (T + 1), cudaMemcpyHostToDevice)))) return done(rc);
+  if (all != m) return fail(TRUST_TC_E_DEVICE);
+  if ((rc = cu(cudaMalloc((void **)&tbase, sizeof(int64_t) * (T + 1))))) return fail(rc);
+  if ((rc = cu(cudaMalloc((void **)&out, sizeof(int32_t) * (size_t)std::max<int64_t>(hbase[T], 1))))) return fail(rc);
+  if ((rc = cu(cudaMemcpy(tbase, hbase.data(), sizeof(int64_t) * (T + 1), cudaMemcpyHostToDevice)))) return fail(rc);
   part_fill_kernel<<<blocks, 256, 0, st>>>(beg, adj, n, p, stride, cnt, tbase, out);
   TC_NOTE_LAUNCH();
-  if ((rc = cu(cudaGetLastError()))) return done(rc);
+  if ((rc = cu(cudaGetLastError())) || (rc = cu(cudaStreamSynchronize(st)))) return fail(rc);
+  cudaFree(tbase);
   for (size_t t = 0; t < T; ++t) {
-    PinnedTile &x = tiles[t];
-    if ((rc = cu(cudaMallocHost((void **)&x.beg, sizeof(int64_t) * (size_t)(x.rows + 1))))) break;
-    if ((rc = cu(cudaMallocHost((void **)&x.adj, sizeof(int32_t) * (size_t)std::max<int64_t>(x.m, 1))))) break;
-    if ((rc = cu(cudaMemcpy(x.beg, cnt + t * stride, sizeof(int64_t) * (size_t)(x.rows + 1), cudaMemcpyDeviceToHost))))
-      break;
-    if (x.m && (rc = cu(cudaMemcpy(x.adj, out + hbase[t], sizeof(int32_t) * (size_t)x.m, cudaMemcpyDeviceToHost))))
-      break;
+    tiles[t].beg = cnt + t * stride;
+    tiles[t].adj = out + hbase[t];
   }
-  if (rc) {
-    for (size_t t = 0; t < T; ++t) {
-      cudaFreeHost(tiles[t].beg);
-      cudaFreeHost(tiles[t].adj);
-      tiles[t] = PinnedTile{};
-    }
-  }
-  return done(rc);
+  *d_beg = cnt;
+  *d_adj = out;
+  return TRUST_TC_OK;
 }
 
 }  // namespace tc

@@ -6,7 +6,9 @@
 // per (i,j,k) job (With-graph-partition/TC.cu:988-994): tables from part(i,j), arcs from
 // part(i,k), probe lists from part(k,j).  Here all parts^3 jobs run on one GPU through the same
 // persistent kernel, with the tiles kept in a device cache bounded by a byte budget so a graph
-// larger than HBM streams its tiles in from host memory.
+// larger than HBM streams its tiles in from host memory.  A device CSR's tiles are made on the GPU:
+// where the budget holds all of them they are the cache, and go to pinned host memory only otherwise
+// (pinning and copying them took 10 of the 34 ms of a call on R-MAT 21 as 2 x 2 tiles: now 23.8).
 #include <cuda_runtime.h>
 #include <errno.h>
 #include <stdio.h>
@@ -24,11 +26,7 @@
 
 namespace {
 
-struct HostTile {
-  int64_t *beg = nullptr;
-  int32_t *adj = nullptr;
-  int64_t rows = 0, m = 0;
-};
+using tc::Tile;
 
 struct DevTile {
   int64_t *beg = nullptr;
@@ -84,23 +82,22 @@ int trust_tc_partition_folder(const char *folder, const int64_t *beg, const int3
 
 namespace tc {
 
-// The (i,j,k) jobs over p x p host tiles (all p*p present, ht[i*p+j]), the tiles kept in a device
-// cache with an LRU byte budget (0 = 80 % of the free memory at entry).  r->call_seconds covers
-// the whole loop including the host-to-device tile copies.
-int tile_loop(const std::vector<HostTile> &ht, int p, const trust_tc_opts &o, size_t budget_bytes,
-              trust_tc_result *r) {
+static size_t cache_budget(size_t budget_bytes, size_t held) {
+  size_t free_b = 0, total_b = 0;
+  if (!budget_bytes) cudaMemGetInfo(&free_b, &total_b);
+  return budget_bytes ? budget_bytes : (free_b + held) / 10 * 8;
+}
+
+// The (i,j,k) jobs over p x p tiles (all p*p present, ht[i*p+j]): host tiles, kept in a device cache
+// with an LRU byte budget (0 = 80 % of the free memory at entry), or - on_device - tiles that already
+// lie on the device and stay the caller's.  r->call_seconds covers the whole loop including any
+// host-to-device tile copies.  The context is the call's own.
+static int tile_loop(trust_tc_ctx &ctx, const std::vector<Tile> &ht, bool on_device, int p, const trust_tc_opts &o,
+                     size_t budget_bytes, trust_tc_result *r) {
   int rc = TRUST_TC_OK;
   int64_t total_m = 0;
   for (const auto &t : ht) total_m += t.m;
-  trust_tc_ctx ctx;
-  rc = ctx_init(&ctx, o.device);
-  if (rc) {
-    ctx_release(&ctx);
-    return rc;
-  }
-  size_t free_b = 0, total_b = 0;
-  cudaMemGetInfo(&free_b, &total_b);
-  const size_t budget = budget_bytes ? budget_bytes : free_b / 10 * 8;
+  const size_t budget = on_device ? 0 : cache_budget(budget_bytes, 0);
   std::vector<DevTile> dt((size_t)p * p);
   std::list<int> lru;
   size_t used = 0;
@@ -117,19 +114,31 @@ int tile_loop(const std::vector<HostTile> &ht, int p, const trust_tc_opts &o, si
     }
     return false;
   };
-  uint64_t copied = 0;
   // per tile: rows strictly increasing (so duplicate-free), checked on its first copy; the
   // direction split of a job needs it of the job's table and probe tiles
   std::vector<signed char> increasing((size_t)p * p, -1);
+  auto known_increasing = [&](int id) -> int {
+    if (increasing[id] >= 0) return TRUST_TC_OK;
+    bool inc = false;
+    const int rc2 = rows_increasing(&ctx, dt[id].beg, dt[id].adj, ht[id].rows, (cudaStream_t)o.stream, &inc);
+    if (!rc2) increasing[id] = inc ? 1 : 0;
+    return rc2;
+  };
   auto fetch = [&](int id, int k0, int k1, int k2) -> int {
     DevTile &d = dt[id];
+    const Tile &h = ht[id];
     if (d.resident) {
       lru.remove(id);
       lru.push_front(id);
       return TRUST_TC_OK;
     }
-    const HostTile &h = ht[id];
-    size_t bytes = sizeof(int64_t) * (size_t)(h.rows + 1) + sizeof(int32_t) * (size_t)std::max<int64_t>(h.m, 1);
+    if (on_device) {
+      d.beg = h.beg;
+      d.adj = h.adj;
+      d.resident = true;
+      return known_increasing(id);
+    }
+    const size_t bytes = h.bytes();
     while (used + bytes > budget && evict_one(k0, k1, k2)) {
     }
     cudaError_t e = cudaMalloc(&d.beg, sizeof(int64_t) * (size_t)(h.rows + 1));
@@ -142,18 +151,11 @@ int tile_loop(const std::vector<HostTile> &ht, int p, const trust_tc_opts &o, si
       d = DevTile();
       return cuda_status(e);
     }
-    copied += bytes;
     d.bytes = bytes;
     d.resident = true;
     used += bytes;
     lru.push_front(id);
-    if (increasing[id] < 0) {
-      bool inc = false;
-      const int rc2 = rows_increasing(&ctx, d.beg, d.adj, h.rows, (cudaStream_t)o.stream, &inc);
-      if (rc2) return rc2;
-      increasing[id] = inc ? 1 : 0;
-    }
-    return TRUST_TC_OK;
+    return known_increasing(id);
   };
   uint64_t *cycles = r->vertex_cycles;
   memset(r, 0, sizeof *r);
@@ -204,18 +206,17 @@ int tile_loop(const std::vector<HostTile> &ht, int p, const trust_tc_opts &o, si
   cudaEventElapsedTime(&ms, e0, e1);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  for (auto &d : dt) {
-    cudaFree(d.beg);
-    cudaFree(d.adj);
-  }
-  ctx_release(&ctx);
+  if (!on_device)
+    for (auto &d : dt) {
+      cudaFree(d.beg);
+      cudaFree(d.adj);
+    }
   r->triangles = total;
   r->kernel_seconds = tk;
   r->count_seconds = tcount;
   r->call_seconds = ms * 1e-3;
   r->vertices = n_total;
   r->edges = total_m;
-  (void)copied;
   return rc;
 }
 
@@ -231,44 +232,53 @@ int trust_tc_count_tiles_device(const int64_t *d_begin, const int32_t *d_adj, in
   trust_tc_opts o;
   if (opts) o = *opts; else trust_tc_opts_init(&o);
   if (o.row_begin || o.row_end) return TRUST_TC_E_UNSUPPORTED;  // row ranges: single-graph calls only
-  int rc = TRUST_TC_OK;
-  {  // validate the whole CSR before the partition reads it
-    trust_tc_ctx ctx;
-    rc = tc::ctx_init(&ctx, o.device);
-    if (!rc) {
-      cudaError_t e = cudaMemset(ctx.d_ctl, 0, sizeof(TcControl));
-      rc = e == cudaSuccess ? tc::launch_check(d_begin, d_adj, n, m, n, 1, ctx.d_ctl, ctx.num_sms, 0)
-                            : tc::cuda_status(e);
-      if (!rc) {
-        e = cudaMemcpy(ctx.h_ctl, ctx.d_ctl, sizeof(TcControl), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) rc = tc::cuda_status(e);
-      }
-      if (!rc) {
-        const int st = ctx.h_ctl->status;
-        if (st & TC_DEV_BAD_OFFSETS) rc = TRUST_TC_E_OFFSETS;
-        else if (st & TC_DEV_TOO_LARGE) rc = TRUST_TC_E_TOO_LARGE;
-        else if (st & TC_DEV_BAD_IDS) rc = TRUST_TC_E_IDS;
-      }
-    }
-    tc::ctx_release(&ctx);
-    if (rc) return rc;
-  }
   const int p = parts;
-  std::vector<tc::PinnedTile> pt((size_t)p * p);
-  rc = tc::partition_device_to_host(d_begin, d_adj, n, m, p, pt.data());
-  if (rc) return rc;
-  std::vector<HostTile> ht((size_t)p * p);
-  for (size_t t = 0; t < pt.size(); ++t) {
-    ht[t].beg = pt[t].beg;
-    ht[t].adj = pt[t].adj;
-    ht[t].rows = pt[t].rows;
-    ht[t].m = pt[t].m;
+  trust_tc_ctx ctx;
+  int64_t *d_tile_beg = nullptr;
+  int32_t *d_tile_adj = nullptr;
+  std::vector<tc::Tile> tiles((size_t)p * p);
+  auto cu = [](cudaError_t e) { return e == cudaSuccess ? TRUST_TC_OK : tc::cuda_status(e); };
+  int rc = tc::ctx_init(&ctx, o.device);
+  // validate the whole CSR before the partition reads it
+  if (!rc) rc = cu(cudaMemset(ctx.d_ctl, 0, sizeof(TcControl)));
+  if (!rc) rc = tc::launch_check(d_begin, d_adj, n, m, n, 1, ctx.d_ctl, ctx.num_sms, 0);
+  if (!rc) rc = cu(cudaMemcpy(ctx.h_ctl, ctx.d_ctl, sizeof(TcControl), cudaMemcpyDeviceToHost));
+  if (!rc) {
+    const int st = ctx.h_ctl->status;
+    if (st & TC_DEV_BAD_OFFSETS) rc = TRUST_TC_E_OFFSETS;
+    else if (st & TC_DEV_TOO_LARGE) rc = TRUST_TC_E_TOO_LARGE;
+    else if (st & TC_DEV_BAD_IDS) rc = TRUST_TC_E_IDS;
   }
-  rc = tc::tile_loop(ht, p, o, device_budget_bytes, r);
-  for (auto &t : pt) {
-    cudaFreeHost(t.beg);
-    cudaFreeHost(t.adj);
+  if (!rc) rc = tc::partition_device(d_begin, d_adj, n, m, p, tiles.data(), &d_tile_beg, &d_tile_adj);
+  if (!rc) {
+    size_t bytes = 0;
+    for (const auto &t : tiles) bytes += t.bytes();
+    const bool fits = bytes <= tc::cache_budget(device_budget_bytes, bytes);
+    std::vector<tc::Tile> host;
+    if (!fits) {  // all tiles to pinned host memory, and the device copies make room
+      host = tiles;
+      for (auto &t : host) t.beg = nullptr, t.adj = nullptr;
+      for (size_t t = 0; t < host.size() && !rc; ++t) {
+        const size_t nb = sizeof(int64_t) * (size_t)(host[t].rows + 1), na = sizeof(int32_t) * (size_t)host[t].m;
+        rc = cu(cudaMallocHost((void **)&host[t].beg, nb));
+        if (!rc) rc = cu(cudaMallocHost((void **)&host[t].adj, std::max<size_t>(na, sizeof(int32_t))));
+        if (!rc) rc = cu(cudaMemcpy(host[t].beg, tiles[t].beg, nb, cudaMemcpyDeviceToHost));
+        if (!rc && na) rc = cu(cudaMemcpy(host[t].adj, tiles[t].adj, na, cudaMemcpyDeviceToHost));
+      }
+      cudaFree(d_tile_beg);
+      cudaFree(d_tile_adj);
+      d_tile_beg = nullptr;
+      d_tile_adj = nullptr;
+    }
+    if (!rc) rc = tc::tile_loop(ctx, fits ? tiles : host, fits, p, o, device_budget_bytes, r);
+    for (auto &t : host) {
+      cudaFreeHost(t.beg);
+      cudaFreeHost(t.adj);
+    }
   }
+  cudaFree(d_tile_beg);
+  cudaFree(d_tile_adj);
+  tc::ctx_release(&ctx);
   return rc;
 }
 
@@ -278,17 +288,22 @@ int trust_tc_count_partitioned(const char *folder, int parts, const trust_tc_opt
   if (opts) o = *opts; else trust_tc_opts_init(&o);
   if (o.row_begin || o.row_end) return TRUST_TC_E_UNSUPPORTED;  // row ranges: single-graph calls only
   const int p = parts;
-  std::vector<HostTile> ht((size_t)p * p);
+  std::vector<Tile> ht((size_t)p * p);
   int rc = TRUST_TC_OK;
   for (int i = 0; i < p && !rc; ++i)
     for (int j = 0; j < p && !rc; ++j) {
-      HostTile &t = ht[(size_t)i * p + j];
+      Tile &t = ht[(size_t)i * p + j];
       rc = trust_tc_load_folder(tile_dir(folder, i, j).c_str(), &t.beg, &t.adj, &t.rows, &t.m);
     }
   for (int i = 0; i < p && !rc; ++i)
     for (int j = 1; j < p && !rc; ++j)
       if (ht[(size_t)i * p + j].rows != ht[(size_t)i * p].rows) rc = TRUST_TC_E_FORMAT;
-  if (!rc) rc = tc::tile_loop(ht, p, o, 0, r);
+  if (!rc) {
+    trust_tc_ctx ctx;
+    rc = tc::ctx_init(&ctx, o.device);
+    if (!rc) rc = tc::tile_loop(ctx, ht, false, p, o, 0, r);
+    tc::ctx_release(&ctx);
+  }
   for (auto &t : ht) {
     free(t.beg);
     free(t.adj);
