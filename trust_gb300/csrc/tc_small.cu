@@ -7,10 +7,12 @@
 // builds the row's bitmap over all ids in shared memory (a probe is one 4-byte load, no hashing) and
 // probes it, four rows at a time, eight lanes each; the last CTA to finish writes the totals
 // straight into the context's pinned control block and clears the accumulators.
-// Calls on GB300, general path / this one, us: R-MAT 8 (1,311 arcs) 79 / 28, R-MAT 16 ef16 (0.9 M)
-// 404 / 162, K_512 191 / 79, Erdos-Renyi 60,000 / 1.9 M arcs 161 / 133, one row of 15,000 entries 828
+// Calls on GB300, general path / this one, us: R-MAT 8 (1,311 arcs) 79 / 27, R-MAT 16 ef16 (0.9 M)
+// 400 / 142, K_512 191 / 79, Erdos-Renyi 60,000 / 1.9 M arcs 161 / 133, one row of 15,000 entries 828
 // / 555.  Small graphs are bound by the launch and the round trip (device time 12 of R-MAT 8's 28 us),
-// R-MAT 16 by the issue of its 94 M probes and the tail of its longest rows.
+// R-MAT 16 by the issue of its 94 M probes.  Every other round of rows goes to the warps in reverse
+// order: with rows longest first a warp then gets about the same work (R-MAT 16 160 -> 142 us, R-MAT
+// 16 ef32 330 -> 244).  Tried and slower: chunks of 64 arcs whatever their rows (181 us).
 #include <algorithm>
 
 #include "tc_count.h"
@@ -32,7 +34,7 @@ struct SmallArgs {
   int check_ids;
   int warp_max, cta_max;
   int splits;   // warps per row
-  int words;    // bitmap words per warp
+  int words;    // bitmap words per warp; the last one stays zero (entries that are no ids)
   TcControl *acc;    // device accumulators, zero between calls (bad_offset_at: CTAs finished)
   TcControl *out;    // pinned host block
 };
@@ -54,6 +56,7 @@ __global__ void __launch_bounds__(SM_THREADS, 6) small_kernel(SmallArgs p) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = lane >> 3, gl = lane & 7;
   unsigned *words = bitmaps + warp * p.words;
+  const unsigned none = (unsigned)p.words - 1;
   for (int i = lane; i < p.words; i += 32) words[i] = 0;
   if (threadIdx.x < 2 * TC_NUM_CLASSES) (&hist[0][0])[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
@@ -65,7 +68,10 @@ __global__ void __launch_bounds__(SM_THREADS, 6) small_kernel(SmallArgs p) {
   unsigned long long hits = 0, wedges = 0;
   int bad = 0, dmax = 0;
   const int tasks = p.n * p.splits, nwarps = gridDim.x * SM_WARPS;
-  for (int t = blockIdx.x * SM_WARPS + warp; t < tasks; t += nwarps) {
+  const int me = blockIdx.x * SM_WARPS + warp;
+  for (int round = 0; round * nwarps < tasks; ++round) {
+    const int t = round * nwarps + (round & 1 ? nwarps - 1 - me : me);
+    if (t >= tasks) continue;
     const int v = t / p.splits, part = t - v * p.splits;
     int b;
     int d = checked_row(p, v, b);
@@ -124,8 +130,7 @@ __global__ void __launch_bounds__(SM_THREADS, 6) small_kernel(SmallArgs p) {
 #pragma unroll
           for (int r = 0; r < 4; ++r) w[r] = k + 8 * r < dj ? (unsigned)tc_ld_nc(p.adj + sj + k + 8 * r) : 0xffffffffu;
 #pragma unroll
-          for (int r = 0; r < 4; ++r)
-            if (w[r] < (unsigned)p.n) h += words[w[r] >> 5] >> (w[r] & 31u) & 1u;
+          for (int r = 0; r < 4; ++r) h += words[min(w[r] >> 5, none)] >> (w[r] & 31u) & 1u;
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) rest &= rest - 1;
@@ -202,13 +207,13 @@ int small_count(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t
   a.cta_max = cta_max;
   // rows of few batches: a warp each; dense graphs: several warps share a row's batches
   a.splits = (int)std::min<int64_t>(8, std::max<int64_t>(1, m / (16 * n)));
-  a.words = (int)((n + 31) / 32);
+  a.words = (int)(n / 32 + 2);
   a.acc = c->d_small;
   a.out = c->h_ctl;
   const int64_t tasks = n * a.splits;
   const size_t smem = sizeof(unsigned) * (size_t)a.words * SM_WARPS;
   TC_CUDA_TRY(cudaFuncSetAttribute(small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(SMALL_MAX_IDS / 8 * SM_WARPS)));
+                                   (int)sizeof(unsigned) * (SMALL_MAX_IDS / 32 + 2) * SM_WARPS));
   const int per_sm = (int)std::min<size_t>(6, (size_t)220 * 1024 / (smem + 1536));  // resident CTAs
   const int blocks = (int)std::min<int64_t>((tasks + SM_WARPS - 1) / SM_WARPS, (int64_t)c->num_sms * per_sm);
   small_kernel<<<blocks, SM_THREADS, smem, st>>>(a);
