@@ -25,10 +25,11 @@ namespace {
 typedef unsigned int u32;
 
 // ---- column popularity -----------------------------------------------------------------------
-// In-degrees of a sample of the arcs: 32 of every 128 consecutive ones.  The order only decides which
-// columns get the popular blocks, never the count, and a quarter of the arcs gives the same order
-// where it matters (R-MAT 20: 0.28 -> 0.09 ms; the atomics on popular columns bound it).
-constexpr int POP_SAMPLE = 4;
+// In-degrees of a sample of the arcs: 32 of every 512 consecutive ones.  The order only decides which
+// columns get the popular blocks, never the count, and a sixteenth of the arcs gives the same order
+// where it matters (R-MAT 20, all arcs / a quarter / a sixteenth: 0.28 / 0.09 / 0.03 ms; the atomics on
+// popular columns bound it.  R-MAT 24 a = 0.70, a quarter / a sixteenth: 44.2 / 43.7 ms per call).
+constexpr int POP_SAMPLE = 16;
 __global__ void indeg_kernel(const int32_t *__restrict__ adj, int64_t m, u32 *__restrict__ indeg) {
   const int64_t groups = (m + 32 * POP_SAMPLE - 1) / (32 * POP_SAMPLE);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x >> 5;
