@@ -153,3 +153,49 @@ def test_device_tiles_at_the_budget(p, room):
     whole = T.count_tiles(beg, adj, p)
     assert r.triangles == whole.triangles == expect
     assert (r.wedges, r.edges, r.vertices, r.class_sizes) == (whole.wedges, whole.edges, whole.vertices, whole.class_sizes)
+
+
+def _rows_csr(rows, n):
+    d = np.array([len(rows.get(v, ())) for v in range(n)], dtype=np.int64)
+    beg = np.concatenate([[0], np.cumsum(d)]).astype(np.int64)
+    adj = np.concatenate([np.asarray(rows[v]) for v in range(n) if v in rows]).astype(np.int32)
+    return beg, adj
+
+
+@pytest.mark.parametrize("kind", ["complete", "random", "tails"])
+@pytest.mark.parametrize("p", [2, 3])
+def test_tile_jobs_with_long_rows(kind, p):
+    """Tile rows longer than the block-bitmap path's bound (128) in either tile of a job, at the bounds
+    of its conversion kernels, and with columns beyond the bitmap; jobs with one tile on both sides
+    (i = k) and with two."""
+    import torch
+    rng = np.random.default_rng(p)
+    if kind == "complete":
+        n = 1100
+        rows = {v: np.arange(v + 1, n) for v in range(n - 1)}
+    elif kind == "random":
+        n = 5000
+        rows = {v: np.unique(rng.integers(v + 1, n, size=rng.choice([3, 40, 300, 420, 1700]))) for v in range(n - 1)}
+    else:
+        n, hubs = 1_000_000, 40
+        rows = {h: np.unique(np.concatenate([np.arange(h + 1, hubs), rng.integers(hubs, n, size=2600),
+                                             np.arange(hubs, hubs + 700)])) for h in range(hubs)}
+        for v in range(hubs, n - 1, 7):
+            rows[v] = np.unique(rng.integers(v + 1, n, size=4))
+    beg, adj = _rows_csr(rows, n)
+    expect = O.count_forward(beg, adj, threads=8)
+    db, da = torch.from_numpy(beg).cuda(), torch.from_numpy(adj).cuda()
+    on = T.count_tiles(db, da, p, direction_split=1)
+    off = T.count_tiles(db, da, p, direction_split=0)
+    assert on.triangles == off.triangles == expect
+    assert on.direction_split >= p * p and on.wedges <= off.wedges
+    # probes: the shorter row of every arc of every job with a table row
+    d = np.zeros((p, n), dtype=np.int64)  # entries of each row per column class
+    src = np.repeat(np.arange(n), np.diff(beg))
+    for j in range(p):
+        d[j] = np.bincount(src[adj % p == j], minlength=n)
+    diag = np.minimum(d[:, src], d[:, adj])
+    for j in range(p):  # a job over one tile skips rows of one entry
+        one = (src % p == j) & (adj % p == j) & (d[j][src] < 2)
+        diag[j][one] = 0
+    assert on.wedges == int(diag.sum())

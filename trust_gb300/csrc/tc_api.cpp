@@ -345,9 +345,10 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
       same && g.min_deg == 2 && g.rows > 0 &&
       (o.direction_split == 1 || (learned && h.max_out_degree >= 64 && g.mA >= TC_LEARNED_MIN_ARCS &&
                                   (!fused || (double)h.long_arcs >= TC_LEARNED_MIN_LONG_FRAC * (double)g.mA)));
-  // with the split, rows longer than BITS_TABLE_MIN are counted as block bitmaps (tc_bits.cu) unless
+  // with the split (of one graph or of a tile job, below), rows longer than BITS_TABLE_MIN are counted as
+  // block bitmaps (tc_bits.cu) unless
   // the caller asks for something of the hash tables' own: cycles, hub clusters, CTA bounds below
-  const bool bits_ok = consider && !o.record_cycles && o.hub_cluster == 0 && !o.test_wait_expiry &&
+  const bool bits_ok = !o.record_cycles && o.hub_cluster == 0 && !o.test_wait_expiry &&
                        cfg.cta_max >= BITS_TABLE_MIN && bits_eligible(g, h.max_out_degree);
   unsigned long long plan_wedges = 0;
   BitsPlan bits;
@@ -396,8 +397,7 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     }
     if (split && bits_ok) {
       plan_wedges = plan.w_min;
-      rc = bits_prepare(c, g.begA, g.adjA, g.rows, g.mA, row_lo, row_hi < 0 ? g.rows : row_hi, plan, h.max_out_degree,
-                        st, &bits);
+      rc = bits_prepare(c, g, row_lo, row_hi < 0 ? g.rows : row_hi, plan, h.max_out_degree, st, &bits);
       if (rc == TRUST_TC_E_NOMEM) split = 0;  // no room for the blocks (allocated first): count unsplit
       else if (rc) return rc;
       use_bits = rc == TRUST_TC_OK;
@@ -410,13 +410,20 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
                           (o.direction_split < 0 && o.schedule == TRUST_TC_SCHED_LEARNED &&
                            h.max_out_degree >= 64 && g.mB >= TC_LEARNED_MIN_ARCS));
   if (consider3) {
-    rc = tile_split_plan(c, g, st);
+    rc = tile_split_plan(c, g, st, bits_ok ? BITS_TABLE_MIN : 0);
     if (rc) return rc;
     TC_CUDA_TRY(cudaStreamSynchronize(st));
     SchedPlan plan{};
     split_plan_read(c, &plan);
     if (plan.overflow) return TRUST_TC_E_DEVICE;
     split = o.direction_split == 1 || split_pays(plan.w_all, plan.w_min, g.mB, g.rows);
+    if (split && bits_ok) {
+      plan_wedges = plan.w_min;
+      rc = bits_prepare(c, g, 0, g.rows, plan, h.max_out_degree, st, &bits);
+      if (rc == TRUST_TC_E_NOMEM) split = 0;  // as for one graph
+      else if (rc) return rc;
+      use_bits = rc == TRUST_TC_OK;
+    }
   }
   // the fused pass's lists stand unless the learned decisions re-classified the rows
   const bool lists_done = fused && !dec;
@@ -529,7 +536,7 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     if (rc) return rc;
   }
   if (use_bits) {
-    rc = bits_launch(c, bits, g.adjA, ctl, st);
+    rc = bits_launch(c, bits, g.adjB, ctl, st);
     if (rc) return rc;
   }
   // a large graph of short rows only: the row-order kernel

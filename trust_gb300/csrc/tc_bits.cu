@@ -10,6 +10,10 @@
 // probe (a = 0.57), 0.26 (a = 0.70).  Columns beyond the bitmap ("tail" entries, the unpopular
 // ones) stay plain ids after the row's blocks and are looked up in a small hash set.
 //
+// A tile job (tables from tile A, arcs of B, probe rows from C) is counted the same way with the rows of A
+// and of C converted under one column order: A's long rows are probed by the C rows of their arcs, C's
+// long rows by the A rows of the arcs moved to them (R-MAT 21 as 2 x 2 tiles 24.1 -> 17.4 ms per call).
+//
 // The rows must be duplicate-free (the split already requires it), so |N+(v) ∩ N+(u)| is the same
 // number from either side and in any column numbering.
 #include <algorithm>
@@ -128,7 +132,7 @@ constexpr int BITS_WARP_ROW = 512;  // rows up to this are converted by a warp, 
 // listed (longs: warp rows from the front, CTA rows from the back).
 __global__ void __launch_bounds__(256) bits_short_kernel(const int64_t *__restrict__ beg, const int32_t *__restrict__ adj,
                                                          int64_t n, const u32 *__restrict__ rank, int nb,
-                                                         u32 *__restrict__ ent, int4 *__restrict__ desc,
+                                                         u32 base_at, u32 *__restrict__ ent, int4 *__restrict__ desc,
                                                          int *__restrict__ longs, u32 *__restrict__ nlongs) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = tc_lanemask_lt();
@@ -187,7 +191,7 @@ __global__ void __launch_bounds__(256) bits_short_kernel(const int64_t *__restri
       if (valid) {
         const unsigned mine = (dj == 32 ? 0xffffffffu : ((1u << dj) - 1u)) << ex;
         const int nd = __popc(lead & mine), pad = (nd + 3) & ~3;
-        const u32 s = row_start(bj, v0 + own);
+        const u32 s = base_at + row_start(bj, v0 + own);
         if (lead >> lane & 1) ent[s + entry_place(__popc(lead & mine & lt), pad >> 2)] = blk << 17 | mask;
         if (tail) ent[s + pad + __popc(tails & mine & lt)] = w;
         if (lane == ex) {
@@ -227,8 +231,9 @@ __device__ __forceinline__ int group_slots(int d) {
 
 // A warp per row of 33..BITS_WARP_ROW entries.
 __global__ void __launch_bounds__(256) bits_warp_kernel(const int64_t *__restrict__ beg, const int32_t *__restrict__ adj,
-                                                        const u32 *__restrict__ rank, int nb, u32 *__restrict__ ent,
-                                                        int4 *__restrict__ desc, const int *__restrict__ longs,
+                                                        const u32 *__restrict__ rank, int nb, u32 base_at,
+                                                        u32 *__restrict__ ent, int4 *__restrict__ desc,
+                                                        const int *__restrict__ longs,
                                                         const u32 *__restrict__ nlongs) {
   __shared__ u32 tabs[8][2 * BITS_WARP_ROW];
   u32 *tab = tabs[threadIdx.x >> 5];
@@ -251,7 +256,7 @@ __global__ void __launch_bounds__(256) bits_warp_kernel(const int64_t *__restric
     }
     nt = __reduce_add_sync(TC_FULL_MASK, nt);
     __syncwarp();
-    const u32 s = row_start(lo, v);
+    const u32 s = base_at + row_start(lo, v);
     int nd = 0;
     for (int k = lane; k < T; k += 32) nd += tab[k] != 0;
     nd = __reduce_add_sync(TC_FULL_MASK, nd);
@@ -281,7 +286,7 @@ __global__ void __launch_bounds__(256) bits_warp_kernel(const int64_t *__restric
 
 // A CTA per longer row (up to BITS_MAX_ROW entries).
 __global__ void __launch_bounds__(512) bits_cta_kernel(const int64_t *__restrict__ beg, const int32_t *__restrict__ adj,
-                                                       int64_t n, const u32 *__restrict__ rank, int nb,
+                                                       int64_t n, const u32 *__restrict__ rank, int nb, u32 base_at,
                                                        u32 *__restrict__ ent, int4 *__restrict__ desc,
                                                        const int *__restrict__ longs, const u32 *__restrict__ nlongs) {
   extern __shared__ u32 tab[];
@@ -316,7 +321,7 @@ __global__ void __launch_bounds__(512) bits_cta_kernel(const int64_t *__restrict
       nd += wcnt[k];
     }
     const int pad = (nd + 3) & ~3;
-    const u32 s = row_start(lo, v);
+    const u32 s = base_at + row_start(lo, v);
     for (int k = lane; k < seg; k += 32) {  // seg >= 64
       const u32 e = tab[k0 + k];
       const unsigned bm = __ballot_sync(TC_FULL_MASK, e != 0);
@@ -339,36 +344,41 @@ __global__ void __launch_bounds__(512) bits_cta_kernel(const int64_t *__restrict
 // (kept arcs) and of the sources of the arcs moved to it (its in-list).  Its list - out-row, then
 // in-list - is cut into units of about `target` probes (an in-list row counts half the table row: it
 // is shorter), of at least 64 list positions.  In-list space is reserved here with one atomic per
-// warp; cnt[t] becomes the in-list's start.
+// warp; cnt[t] becomes the in-list's start.  A tile job's tables lie in two CSRs: its A rows (side 0)
+// have the rows of B as their out-lists (beg_list) and no in-lists, its C rows (side 1) only in-lists.
 struct Unit {
   int t, lo, hi, len_a;
   u32 a0, b0;
-  int pad0, pad1;
+  int side, pad;
 };
 
-__global__ void __launch_bounds__(256) bits_units_kernel(const int64_t *__restrict__ beg, int64_t n, int64_t row_lo,
+__global__ void __launch_bounds__(256) bits_units_kernel(const int64_t *__restrict__ beg,
+                                                         const int64_t *__restrict__ beg_list, int64_t n, int64_t row_lo,
                                                          int64_t row_hi, int table_min, u32 *__restrict__ cnt,
                                                          const unsigned long long *__restrict__ wsum, u32 *ctr,
-                                                         unsigned long long target, Unit *__restrict__ units) {
+                                                         unsigned long long target, Unit *__restrict__ units, int side) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = tc_lanemask_lt();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t v0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); v0 < n; v0 += stride) {
     const int64_t v = v0 + lane;
     int d = 0;
-    long long b = 0;
-    if (v < n) {
-      b = tc_ld_nc(beg + v);
-      d = (int)(tc_ld_nc(beg + v + 1) - b);
-    }
+    if (v < n) d = (int)(tc_ld_nc(beg + v + 1) - tc_ld_nc(beg + v));
     const bool table = d > table_min;
     if (!__any_sync(TC_FULL_MASK, table)) continue;
-    const u32 nb = table ? cnt[v] : 0u;
-    const int na = table && v >= row_lo && v < row_hi ? d : 0;
+    const u32 nb = table && cnt ? cnt[v] : 0u;
+    long long b = 0;
+    int na = 0;
+    if (table && beg_list && v >= row_lo && v < row_hi) {
+      b = tc_ld_nc(beg_list + v);
+      na = (int)(tc_ld_nc(beg_list + v + 1) - b);
+    }
     const u32 len = nb + (u32)na;
     int k = 0;
     if (len) {
-      const unsigned long long w = wsum[v] + (unsigned long long)nb * (unsigned)d / 2;
+      // (without work sums the out-list's rows count half the table row too)
+      const unsigned long long w = (wsum ? wsum[v] : (unsigned long long)na * (unsigned)d / 2) +
+                                   (unsigned long long)nb * (unsigned)d / 2;
       const unsigned long long kk = max((w + target - 1) / target, 1ull);
       k = (int)min(kk, (unsigned long long)((len + 63) / 64));
     }
@@ -391,10 +401,10 @@ __global__ void __launch_bounds__(256) bits_units_kernel(const int64_t *__restri
     }
     ab = __shfl_sync(TC_FULL_MASK, ab, 31) + sb - nb;
     ak = __shfl_sync(TC_FULL_MASK, ak, 31) + (u32)(sk - k);
-    if (table) cnt[v] = ab;
+    if (table && cnt) cnt[v] = ab;
     const u32 per = k ? (len + k - 1) / k : 0;
     for (int j = 0; j < k; ++j)
-      units[ak + j] = Unit{(int)v, (int)min((u32)j * per, len), (int)min((u32)(j + 1) * per, len), na, (u32)b, ab, 0, 0};
+      units[ak + j] = Unit{(int)v, (int)min((u32)j * per, len), (int)min((u32)(j + 1) * per, len), na, (u32)b, ab, side, 0};
     (void)lt;
   }
 }
@@ -407,7 +417,7 @@ __device__ __forceinline__ u32 tail_hash(u32 w) { return w * 0x9E3779B1u >> (32 
 
 struct BitsArgs {
   const int32_t *adj, *adj_b;
-  const int4 *desc;
+  const int4 *desc, *desc_c;  // rows of A and of C (one graph: the same)
   const u32 *ent;
   const Unit *units;
   u32 *ctr;  // [0] units, [2] claim head
@@ -469,7 +479,7 @@ __global__ void __launch_bounds__(THREADS, MINB) bits_count_kernel(BitsArgs p) {
     const u32 x = atomicAdd(p.ctr + 2, 1u);
     if (x < n_units) {
       su[at] = p.units[x];
-      sd[at] = p.desc[su[at].t];
+      sd[at] = (su[at].side ? p.desc_c : p.desc)[su[at].t];
     } else {
       su[at].t = -1;
     }
@@ -516,7 +526,7 @@ __global__ void __launch_bounds__(THREADS, MINB) bits_count_kernel(BitsArgs p) {
       };
       auto fetch = [&](int id, bool in_a) -> int4 {
         if (id < 0) return make_int4(0, 0, 0, 0);
-        int4 q = __ldg(p.desc + id);
+        int4 q = __ldg((in_a ? p.desc_c : p.desc) + id);
         if (in_a && q.w > td.w) q = make_int4(0, 0, 0, 0);  // counted from that row's side
         return q;
       };
@@ -619,71 +629,105 @@ int blocks_for(int64_t work, int64_t per, int num_sms, int most_per_sm) {
 
 }  // namespace
 
+static bool one_csr(const DevGraph3 &g) { return g.begA == g.begC && g.adjA == g.adjC; }
+
 bool bits_eligible(const DevGraph3 &g, int64_t max_out_degree) {
-  return max_out_degree > BITS_TABLE_MIN && max_out_degree <= BITS_MAX_ROW && g.mA + 6 * g.rows + 8 < ((int64_t)1 << 32);
+  const int64_t words = g.mA + 6 * g.rows + 12 + (one_csr(g) ? 0 : g.mC + 6 * g.rowsC + 12);
+  return max_out_degree > BITS_TABLE_MIN && max_out_degree <= BITS_MAX_ROW && words < ((int64_t)1 << 32);
 }
 
 // Enqueue the conversion and the work units (after the scheduling pass and its readback).
-int bits_prepare(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, int64_t row_lo,
-                 int64_t row_hi, const SchedPlan &plan, int64_t max_out_degree, cudaStream_t st, BitsPlan *out) {
-  const int nb = (int)std::min<int64_t>((((n + 15) / 16) + 7) & ~7ll, BITS_MAX_BLOCKS);
-  const u32 ntiles = (u32)((n + RK_TILE - 1) / RK_TILE);
+int bits_prepare(trust_tc_ctx *c, const DevGraph3 &g, int64_t row_lo, int64_t row_hi, const SchedPlan &plan,
+                 int64_t max_out_degree, cudaStream_t st, BitsPlan *out) {
+  const bool tile = g.begA != g.begB || g.adjA != g.adjB || !one_csr(g);
+  const bool two = !one_csr(g);  // rows of two CSRs are converted
+  const int64_t cols = tile ? g.boundA : g.rows;
+  const int nb = (int)std::min<int64_t>((((cols + 15) / 16) + 7) & ~7ll, BITS_MAX_BLOCKS);
+  const u32 ntiles = (u32)((cols + RK_TILE - 1) / RK_TILE);
   // units: every table at least one, and one more per `target` probes: about eight units per resident
   // CTA, so the last ones end together, but not so small that a unit's set-up shows (R-MAT 18: 1.63 ms
   // at 2^18 probes, 1.81 at 2^20; R-MAT 25: 426 and 415)
   const unsigned long long target = std::min<unsigned long long>(
       std::max<unsigned long long>(plan.w_min / (unsigned long long)(c->num_sms * BITS_MINB * 8), 1ull << 16), 1ull << 20);
-  // list positions are at most 2 m: a unit per table and per 64 of them
-  const int64_t max_units = m / (BITS_TABLE_MIN + 1) + 2 * m / 64 + 1;
+  // list positions are at most 2 mB: a unit per table and per 64 of them
+  const int64_t max_units = (g.mA + (tile ? g.mC : 0)) / (BITS_TABLE_MIN + 1) + 2 * g.mB / 64 + 2;
+  const int64_t rows_c = two ? g.rowsC : 0;
+  const u32 base_c = (u32)((g.mA + 6 * g.rows + 11) & ~3ll);
+  const size_t words = two ? (size_t)base_c + (size_t)(g.mC + 6 * g.rowsC + 8) : (size_t)(g.mA + 6 * g.rows + 8);
   // one scratch block: in-degrees, ranks, rank histogram, counters, row lists
-  const size_t nn = (size_t)n;
+  const size_t nn = (size_t)cols;
   const size_t hist = 256 * (size_t)ntiles;
   int rc;
   if ((rc = ensure((void **)&c->d_bits_cols, &c->bits_cols_cap,
-                   sizeof(u32) * (3 * nn + hist + scan_u32_scratch(256 * (int64_t)ntiles) + 16))))
+                   sizeof(u32) * (2 * nn + (size_t)std::max(g.rows, rows_c) + hist +
+                                  scan_u32_scratch(256 * (int64_t)ntiles) + 16))))
     return rc;
-  if ((rc = ensure((void **)&c->d_bits_desc, &c->bits_desc_cap, sizeof(int4) * nn))) return rc;
-  if ((rc = ensure((void **)&c->d_bits_ent, &c->bits_ent_cap, sizeof(u32) * (size_t)(m + 6 * n + 8)))) return rc;
+  if ((rc = ensure((void **)&c->d_bits_desc, &c->bits_desc_cap, sizeof(int4) * (size_t)(g.rows + rows_c)))) return rc;
+  if ((rc = ensure((void **)&c->d_bits_ent, &c->bits_ent_cap, sizeof(u32) * words))) return rc;
   if ((rc = ensure((void **)&c->d_bits_units, &c->bits_units_cap, sizeof(Unit) * (size_t)max_units))) return rc;
-  if ((rc = ensure((void **)&c->d_split_adj, &c->split_adj_cap, sizeof(int32_t) * (size_t)std::max<int64_t>(m, 1))))
+  if ((rc = ensure((void **)&c->d_split_adj, &c->split_adj_cap, sizeof(int32_t) * (size_t)std::max<int64_t>(g.mB, 1))))
     return rc;
   u32 *indeg = c->d_bits_cols, *rank = indeg + nn, *counts = rank + nn;
   u32 *scratch = counts + hist;
-  u32 *ctr = scratch + scan_u32_scratch(256 * (int64_t)ntiles);  // units, in-list entries, claims, warp rows, CTA rows
+  // units, in-list entries, claims, then warp rows and CTA rows of either CSR
+  u32 *ctr = scratch + scan_u32_scratch(256 * (int64_t)ntiles);
   int *longs = reinterpret_cast<int *>(ctr + 16);
   int4 *desc = reinterpret_cast<int4 *>(c->d_bits_desc);
+  int4 *desc_c = two ? desc + g.rows : desc;
   Unit *units = reinterpret_cast<Unit *>(c->d_bits_units);
   TC_CUDA_TRY(cudaMemsetAsync(indeg, 0, sizeof(u32) * nn, st));
   TC_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(u32) * 16, st));
-  indeg_kernel<<<blocks_for(m, 1024, c->num_sms, 16), 256, 0, st>>>(adj, m, indeg);
-  rank_hist_kernel<<<ntiles, 256, 0, st>>>(indeg, n, counts, ntiles);
-  TC_CUDA_TRY(cudaGetLastError());
-  note_launch(2);
-  if ((rc = scan_exclusive_u32(counts, counts, 256 * (int64_t)ntiles, scratch, st))) return rc;
-  rank_scatter_kernel<<<ntiles, 256, 0, st>>>(indeg, n, counts, ntiles, rank);
-  bits_short_kernel<<<blocks_for(n, 256, c->num_sms, 32), 256, 0, st>>>(beg, adj, n, rank, nb, c->d_bits_ent, desc,
-                                                                        longs, ctr + 3);
-  bits_warp_kernel<<<c->num_sms * 7, 256, 0, st>>>(beg, adj, rank, nb, c->d_bits_ent, desc, longs, ctr + 3);
-  note_launch(3);
-  TC_CUDA_TRY(cudaGetLastError());
-  if (max_out_degree > BITS_WARP_ROW) {
-    int T = 64;
-    while (T < 2 * max_out_degree) T <<= 1;
-    const int smem = 4 * T;
-    TC_CUDA_TRY(cudaFuncSetAttribute(bits_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 2 * BITS_MAX_ROW));
-    bits_cta_kernel<<<c->num_sms * std::min(4, (int)(200 * 1024 / (smem + 2048))), 512, smem, st>>>(
-        beg, adj, n, rank, nb, c->d_bits_ent, desc, longs, ctr + 3);
-    note_launch();
-    TC_CUDA_TRY(cudaGetLastError());
-  }
-  bits_units_kernel<<<blocks_for(n, 256, c->num_sms, 16), 256, 0, st>>>(beg, n, row_lo, row_hi, BITS_TABLE_MIN,
-                                                                        c->d_split_cnt, c->d_split_wsum, ctr, target,
-                                                                        units);
+  indeg_kernel<<<blocks_for(g.mA, 1024, c->num_sms, 16), 256, 0, st>>>(g.adjA, g.mA, indeg);
   note_launch();
+  if (two) {
+    indeg_kernel<<<blocks_for(g.mC, 1024, c->num_sms, 16), 256, 0, st>>>(g.adjC, g.mC, indeg);
+    note_launch();
+  }
+  rank_hist_kernel<<<ntiles, 256, 0, st>>>(indeg, cols, counts, ntiles);
   TC_CUDA_TRY(cudaGetLastError());
-  if ((rc = split_fill_u32(c, m, c->d_split_cnt, st))) return rc;
+  note_launch();
+  if ((rc = scan_exclusive_u32(counts, counts, 256 * (int64_t)ntiles, scratch, st))) return rc;
+  rank_scatter_kernel<<<ntiles, 256, 0, st>>>(indeg, cols, counts, ntiles, rank);
+  note_launch();
+  auto convert = [&](const int64_t *beg, const int32_t *adj, int64_t n, u32 base, int4 *d, u32 *nlongs) -> int {
+    bits_short_kernel<<<blocks_for(n, 256, c->num_sms, 32), 256, 0, st>>>(beg, adj, n, rank, nb, base, c->d_bits_ent, d,
+                                                                          longs, nlongs);
+    bits_warp_kernel<<<c->num_sms * 7, 256, 0, st>>>(beg, adj, rank, nb, base, c->d_bits_ent, d, longs, nlongs);
+    note_launch(2);
+    TC_CUDA_TRY(cudaGetLastError());
+    if (max_out_degree > BITS_WARP_ROW) {
+      int T = 64;
+      while (T < 2 * max_out_degree) T <<= 1;
+      const int smem = 4 * T;
+      TC_CUDA_TRY(
+          cudaFuncSetAttribute(bits_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 2 * BITS_MAX_ROW));
+      bits_cta_kernel<<<c->num_sms * std::min(4, (int)(200 * 1024 / (smem + 2048))), 512, smem, st>>>(
+          beg, adj, n, rank, nb, base, c->d_bits_ent, d, longs, nlongs);
+      note_launch();
+      TC_CUDA_TRY(cudaGetLastError());
+    }
+    return TRUST_TC_OK;
+  };
+  if ((rc = convert(g.begA, g.adjA, g.rows, 0, desc, ctr + 3))) return rc;
+  if (two && (rc = convert(g.begC, g.adjC, g.rowsC, base_c, desc_c, ctr + 5))) return rc;
+  const auto cut = [&](const int64_t *beg, const int64_t *beg_list, int64_t n, u32 *cnt, const unsigned long long *wsum,
+                       int side) {
+    bits_units_kernel<<<blocks_for(n, 256, c->num_sms, 16), 256, 0, st>>>(beg, beg_list, n, row_lo, row_hi,
+                                                                          BITS_TABLE_MIN, cnt, wsum, ctr, target, units,
+                                                                          side);
+    note_launch();
+  };
+  if (tile) {
+    cut(g.begA, g.begB, g.rows, nullptr, nullptr, 0);
+    cut(g.begC, nullptr, g.rowsC, c->d_split_cnt, nullptr, 1);
+  } else {
+    cut(g.begA, g.begA, g.rows, c->d_split_cnt, c->d_split_wsum, 0);
+  }
+  TC_CUDA_TRY(cudaGetLastError());
+  if ((rc = split_fill_u32(c, g.mB, c->d_split_cnt, st))) return rc;
   out->nb = nb;
   out->ctr = ctr;
+  out->rows_c_at = two ? g.rows : 0;
   return TRUST_TC_OK;
 }
 
@@ -692,6 +736,7 @@ int bits_launch(trust_tc_ctx *c, const BitsPlan &plan, const int32_t *adj, TcCon
   a.adj = adj;
   a.adj_b = c->d_split_adj;
   a.desc = reinterpret_cast<const int4 *>(c->d_bits_desc);
+  a.desc_c = a.desc + plan.rows_c_at;
   a.ent = c->d_bits_ent;
   a.units = reinterpret_cast<const Unit *>(c->d_bits_units);
   a.ctr = plan.ctr;

@@ -14,13 +14,14 @@ constexpr int BITS_MAX_ROW = 8192;
 struct BitsPlan {
   int nb = 0;               // blocks (of 16 columns) of the bitmap
   unsigned *ctr = nullptr;  // device counters: units, in-list entries, unit claims
+  int64_t rows_c_at = 0;    // first C row among the row descriptors
 };
 
 bool bits_eligible(const DevGraph3 &g, int64_t max_out_degree);
-// After the scheduling pass (its pairs, counts and work sums) and its readback.  Only arcs of
-// source rows in [row_lo, row_hi) are counted.
-int bits_prepare(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, int64_t row_lo,
-                 int64_t row_hi, const SchedPlan &plan, int64_t max_out_degree, cudaStream_t st, BitsPlan *out);
+// After the scheduling pass (its pairs, counts and, for one graph, work sums) and its readback.  Only arcs
+// of source rows in [row_lo, row_hi) are counted.  A tile job's A and C rows must be duplicate-free.
+int bits_prepare(trust_tc_ctx *c, const DevGraph3 &g, int64_t row_lo, int64_t row_hi, const SchedPlan &plan,
+                 int64_t max_out_degree, cudaStream_t st, BitsPlan *out);
 int bits_launch(trust_tc_ctx *c, const BitsPlan &plan, const int32_t *adj, TcControl *ctl, cudaStream_t st);
 
 }  // namespace tc

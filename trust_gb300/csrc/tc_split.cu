@@ -554,14 +554,15 @@ void split_plan_read(const trust_tc_ctx *c, SchedPlan *plan) {
 // A tile job (i,j,k) hashes table rows A[v] (tile (i,j)), walks the arcs (v,u) of B[v] (tile
 // (i,k)) and streams probe rows C[u] (tile (k,j)); an arc costs |C[u]| probes.  Counted from u's
 // side (hash C[u], stream A[v]) it costs |A[v]|, and |A[v] ∩ C[u]| is the same number when both
-// rows are duplicate-free.  The plan moves every arc with |C[u]| > |A[v]| of a row with A[v]
+// rows are duplicate-free.  The plan moves every arc with |C[u]| > max(|A[v]|, table_min) of a row with A[v]
 // nonempty (rows with A[v] empty contribute nothing from either side).  Tile rows are short (a
 // quarter of a 2x2 split's row on average), so a warp takes 32 rows per step, as the whole-graph
 // pass does.
 __global__ void tile_sched_kernel(const int64_t *__restrict__ begA, const int64_t *__restrict__ begB,
                                   const int32_t *__restrict__ adjB, const int64_t *__restrict__ begC, int64_t rows,
                                   unsigned *__restrict__ cnt, unsigned long long *__restrict__ wsum,
-                                  unsigned long long *plans, PairArrays pairs, unsigned long long pair_cap) {
+                                  unsigned long long *plans, PairArrays pairs, unsigned long long pair_cap,
+                                  int table_min) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -578,7 +579,8 @@ __global__ void tile_sched_kernel(const int64_t *__restrict__ begA, const int64_
       w_all += (unsigned)du;
       w_min += (unsigned)min(du, dA);
     }
-    move_arc(valid && du > dA, u, v, dA, cnt, wsum, pairs, plans + PLAN_NPAIRS, pb);
+    move_arc(valid && du > max(dA, table_min), u, v, dA, cnt, table_min ? nullptr : wsum, pairs, plans + PLAN_NPAIRS,
+             pb);
   };
   // 32 consecutive rows per warp step: rows of up to 32 arcs flattened over the lanes (owner from
   // a start-bit mask, as in the whole-graph pass), longer rows walked by the warp one at a time
@@ -641,7 +643,7 @@ __global__ void tile_sched_kernel(const int64_t *__restrict__ begA, const int64_
   }
 }
 
-int tile_split_plan(trust_tc_ctx *c, const DevGraph3 &g, cudaStream_t st) {
+int tile_split_plan(trust_tc_ctx *c, const DevGraph3 &g, cudaStream_t st, int table_min) {
   const size_t nt = (size_t)std::max<int64_t>(g.rowsC + 1, 1);  // targets u: rows of C
   int rc = ensure((void **)&c->d_split_cnt, &c->split_cnt_cap, sizeof(unsigned) * nt);
   if (rc) return rc;
@@ -656,7 +658,7 @@ int tile_split_plan(trust_tc_ctx *c, const DevGraph3 &g, cudaStream_t st) {
   TC_CUDA_TRY(cudaMemsetAsync(c->d_split_wsum, 0, sizeof(unsigned long long) * nt, st));
   TC_CUDA_TRY(cudaMemsetAsync(c->d_split_plans, 0, TC_PLAN_WORDS * sizeof(unsigned long long), st));
   tile_sched_kernel<<<blocks, 256, 0, st>>>(g.begA, g.begB, g.adjB, g.begC, g.rows, c->d_split_cnt, c->d_split_wsum,
-                                            c->d_split_plans, pairs, slots);
+                                            c->d_split_plans, pairs, slots, table_min);
   TC_NOTE_LAUNCH();
   TC_CUDA_TRY(cudaGetLastError());
   TC_CUDA_TRY(cudaMemcpyAsync(c->h_plans, c->d_split_plans, TC_PLAN_WORDS * sizeof(unsigned long long),
