@@ -353,6 +353,20 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
   unsigned long long plan_wedges = 0;
   BitsPlan bits;
   bool use_bits = false;
+  // The conversion to blocks and their counting run on the context's second stream (all they read is
+  // complete: the host has read the scheduling pass's totals) while this one counts the short rows: the
+  // conversion and the short rows both wait on loads, and each fills the other's last wave.
+  struct SideStream {
+    cudaStream_t stream = nullptr;
+    ~SideStream() {  // an early return leaves nothing running on the context's buffers
+      if (stream) cudaStreamSynchronize(stream);
+    }
+  } side;
+  auto prepare_bits = [&](int64_t lo, int64_t hi, const SchedPlan &plan) -> int {
+    if (!c->sub_stream) TC_CUDA_TRY(cudaStreamCreateWithFlags(&c->sub_stream, cudaStreamNonBlocking));
+    side.stream = c->sub_stream;
+    return bits_prepare(c, g, lo, hi, plan, h.max_out_degree, c->sub_stream, &bits);
+  };
   if (consider) {
     const float *d_model = nullptr;
     if (learned) {
@@ -397,7 +411,7 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     }
     if (split && bits_ok) {
       plan_wedges = plan.w_min;
-      rc = bits_prepare(c, g, row_lo, row_hi < 0 ? g.rows : row_hi, plan, h.max_out_degree, st, &bits);
+      rc = prepare_bits(row_lo, row_hi < 0 ? g.rows : row_hi, plan);
       if (rc == TRUST_TC_E_NOMEM) split = 0;  // no room for the blocks (allocated first): count unsplit
       else if (rc) return rc;
       use_bits = rc == TRUST_TC_OK;
@@ -419,7 +433,7 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     split = o.direction_split == 1 || split_pays(plan.w_all, plan.w_min, g.mB, g.rows);
     if (split && bits_ok) {
       plan_wedges = plan.w_min;
-      rc = bits_prepare(c, g, 0, g.rows, plan, h.max_out_degree, st, &bits);
+      rc = prepare_bits(0, g.rows, plan);
       if (rc == TRUST_TC_E_NOMEM) split = 0;  // as for one graph
       else if (rc) return rc;
       use_bits = rc == TRUST_TC_OK;
@@ -536,8 +550,9 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     if (rc) return rc;
   }
   if (use_bits) {
-    rc = bits_launch(c, bits, g.adjB, ctl, st);
+    rc = bits_launch(c, bits, g.adjB, ctl, c->sub_stream);
     if (rc) return rc;
+    TC_CUDA_TRY(cudaEventRecord(c->ev_split[0], c->sub_stream));
   }
   // a large graph of short rows only: the row-order kernel
   const bool short_rows = same && !g.rowmap && g.min_deg == 2 && o.schedule != TRUST_TC_SCHED_PLAIN && !o.record_cycles &&
@@ -547,6 +562,10 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
   else
     rc = launch_count(same, a, blocks, cfg.threads, smem, st);
   if (rc) return rc;
+  if (use_bits) {
+    TC_CUDA_TRY(cudaStreamWaitEvent(st, c->ev_split[0], 0));
+    side.stream = nullptr;
+  }
   TC_CUDA_TRY(cudaEventRecord(c->ev[3], st));
   TC_CUDA_TRY(cudaMemcpyAsync(c->h_ctl, ctl, sizeof(TcControl), cudaMemcpyDeviceToHost, st));
   trust_tc_result rb;
