@@ -8,7 +8,7 @@
 // persistent kernel, with the tiles kept in a device cache bounded by a byte budget so a graph
 // larger than HBM streams its tiles in from host memory.  A device CSR's tiles are made on the GPU:
 // where the budget holds all of them they are the cache, and go to pinned host memory only otherwise
-// (pinning and copying them took 10 of the 34 ms of a call on R-MAT 21 as 2 x 2 tiles: now 23.8).
+// (pinning and copying them took 10 of the 34 ms of a call on R-MAT 21 as 2 x 2 tiles).
 #include <cuda_runtime.h>
 #include <errno.h>
 #include <stdio.h>
