@@ -8,12 +8,13 @@
 // probes it, four rows at a time, eight lanes each; the last CTA to finish writes the totals
 // straight into the context's pinned control block and clears the accumulators.
 // Calls on GB300, general path / this one, us: R-MAT 8 (1,311 arcs) 79 / 27, R-MAT 16 ef16 (0.9 M)
-// 400 / 142, K_512 191 / 79, Erdos-Renyi 60,000 / 1.9 M arcs 161 / 133, one row of 15,000 entries 828
+// 400 / 126, K_512 191 / 79, Erdos-Renyi 60,000 / 1.9 M arcs 161 / 133, one row of 15,000 entries 828
 // / 555.  Small graphs are bound by the launch and the round trip (device time 12 of R-MAT 8's 28 us),
 // R-MAT 16 by the issue of its 94 M probes.  Every other round of rows goes to the warps in reverse
 // order: with rows longest first a warp then gets about the same work (R-MAT 16 160 -> 142 us, R-MAT
 // 16 ef32 330 -> 244).  Tried and slower: chunks of 64 arcs whatever their rows (181 us).
 #include <algorithm>
+#include <type_traits>
 
 #include "tc_count.h"
 #include "tc_internal.h"
@@ -115,7 +116,9 @@ __global__ void __launch_bounds__(SM_THREADS, 6) small_kernel(SmallArgs p) {
       if (!counted) continue;
       wedges += (unsigned)dd;
       unsigned h = 0;
-      // four rows at a time, eight lanes each
+      // four rows at a time, eight lanes each: 64 entries of each per step while one has more than 32 left
+      // (R-MAT 16 ef16 142 -> 126 us, ef28 261 -> 227), else 32
+      const bool longer = __any_sync(TC_FULL_MASK, dd > 32);
       const unsigned have = __ballot_sync(TC_FULL_MASK, dd > 0);
       for (unsigned rest = have; rest;) {
         // the grp-th remaining row
@@ -125,13 +128,18 @@ __global__ void __launch_bounds__(SM_THREADS, 6) small_kernel(SmallArgs p) {
         const int sj = __shfl_sync(TC_FULL_MASK, s, j);
         int dj = __shfl_sync(TC_FULL_MASK, dd, j);
         if (!mine) dj = 0;
-        for (int k = gl; __any_sync(TC_FULL_MASK, k < dj); k += 32) {
-          unsigned w[4];
+        auto walk = [&](int k, auto steps) {
+          constexpr int U = decltype(steps)::value;
+          unsigned w[U];
 #pragma unroll
-          for (int r = 0; r < 4; ++r) w[r] = k + 8 * r < dj ? (unsigned)tc_ld_nc(p.adj + sj + k + 8 * r) : 0xffffffffu;
+          for (int r = 0; r < U; ++r) w[r] = k + 8 * r < dj ? (unsigned)tc_ld_nc(p.adj + sj + k + 8 * r) : 0xffffffffu;
 #pragma unroll
-          for (int r = 0; r < 4; ++r) h += words[min(w[r] >> 5, none)] >> (w[r] & 31u) & 1u;
-        }
+          for (int r = 0; r < U; ++r) h += words[min(w[r] >> 5, none)] >> (w[r] & 31u) & 1u;
+        };
+        int k = gl;
+        if (longer)
+          for (; __any_sync(TC_FULL_MASK, k + 32 < dj); k += 64) walk(k, std::integral_constant<int, 8>());
+        for (; __any_sync(TC_FULL_MASK, k < dj); k += 32) walk(k, std::integral_constant<int, 4>());
 #pragma unroll
         for (int k = 0; k < 4; ++k) rest &= rest - 1;
       }
