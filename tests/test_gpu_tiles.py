@@ -199,3 +199,26 @@ def test_tile_jobs_with_long_rows(kind, p):
         one = (src % p == j) & (adj % p == j) & (d[j][src] < 2)
         diag[j][one] = 0
     assert on.wedges == int(diag.sum())
+
+
+@pytest.mark.parametrize("arcs,table", [(5000, 50), (5000, 128), (5000, 129), (4097, 1), (8192, 60)])
+def test_plain_schedule_tile_rows_long_in_arcs_alone(arcs, table):
+    """Under the plain schedule a tile row's class follows the longer of its table and its arcs: rows of
+    many arcs (huge class) and a short table are counted with the split as without it."""
+    import torch
+    n = 40_000
+    rng = np.random.default_rng(arcs + table)
+    rows = {v: np.unique(rng.integers(v + 1, n, size=rng.choice([2, 30, 70, 150]))) for v in range(n // 2)}
+    odd, even = np.arange(1, n, 2), np.arange(2, n, 2)
+    for v in (0, 1, 2):  # `arcs` entries in one column class, `table` in the other
+        many, few = (odd, even) if v == 1 else (even, odd)
+        rows[v] = np.unique(np.concatenate([rng.choice(many[many > 2], arcs, replace=False),
+                                            rng.choice(few[few > 2], table, replace=False)]))
+    beg, adj = _rows_csr(rows, n)
+    expect = O.count_forward(beg, adj, threads=8)
+    db, da = torch.from_numpy(beg).cuda(), torch.from_numpy(adj).cuda()
+    for schedule in (T.SCHED_PLAIN, T.SCHED_TUNED):
+        on = T.count_tiles(db, da, 2, schedule=schedule, direction_split=1)
+        off = T.count_tiles(db, da, 2, schedule=schedule, direction_split=0)
+        assert on.triangles == off.triangles == expect
+        assert on.direction_split >= 1 and on.class_sizes == off.class_sizes

@@ -494,7 +494,8 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
   // table's bytes then also hold a 512-byte overflow list (tc_count.cu, TC_Q16_OVERFLOW)
   const int key_bits = ceil_log2_size(std::max<int64_t>(std::max(g.boundA, g.boundC), 2));
   const bool q16 = key_bits <= 26;
-  if (h.class_count[TC_CLASS_CTA] > 0) {
+  // (with block bitmaps, huge rows with short tables are counted like CTA rows)
+  if (h.class_count[TC_CLASS_CTA] > 0 || (use_bits && h.class_count[TC_CLASS_HUGE] > 0)) {
     const int64_t dcta = std::min<int64_t>(use_bits ? longest : h.max_out_degree, cfg.cta_max);
     smem = std::max(smem, ((size_t)4 << std::max(ceil_log2_size(2 * dcta), 6)) + (q16 ? 512 : 0));
   }

@@ -1022,11 +1022,14 @@ __global__ void __launch_bounds__(MAXT, MINB) count_kernel(CountArgs p) {
   // Phase A: CTA-granularity vertices, largest class first.
   for (int c = TC_CLASS_HUGE; c >= TC_CLASS_CTA; --c) {
     const int n_items = p.ctl->class_count[c];
-    if (n_items == 0 || (c == TC_CLASS_HUGE && p.table_min > 0)) continue;
-    if (c == TC_CLASS_HUGE && (int)blockIdx.x >= p.huge_blocks) continue;
+    // With block bitmaps only rows with tables of up to table_min entries are counted here: none of one
+    // CSR's huge rows, but a tile job's row may be huge for its arcs alone (plain split: the longer of
+    // both decides), and its table then fits shared memory.
+    if (n_items == 0 || (SAME && c == TC_CLASS_HUGE && p.table_min > 0)) continue;
+    const bool spill = c == TC_CLASS_HUGE && p.table_min == 0;
+    if (spill && (int)blockIdx.x >= p.huge_blocks) continue;
     const int *list = class_list(p, c);
-    int *tab = (c == TC_CLASS_HUGE) ? p.huge_tables + (size_t)blockIdx.x * ((size_t)1 << p.huge_log2)
-                                    : smem;
+    int *tab = spill ? p.huge_tables + (size_t)blockIdx.x * ((size_t)1 << p.huge_log2) : smem;
     for (;;) {
       __syncthreads();
       if (threadIdx.x == 0) bs.item = atomicAdd(&p.ctl->class_next[c], 1);
@@ -1045,7 +1048,7 @@ __global__ void __launch_bounds__(MAXT, MINB) count_kernel(CountArgs p) {
         if (d > p.table_min) continue;
       }
       const long long t_start = REC ? clock64() : 0;
-      cta_vertex<SAME>(p, v, tab, c == TC_CLASS_CTA, bs, hits, wedges);
+      cta_vertex<SAME>(p, v, tab, !spill, bs, hits, wedges);
       if (REC && threadIdx.x == 0) p.cycles[v] = (unsigned long long)(clock64() - t_start);
     }
   }
