@@ -83,3 +83,52 @@ def test_longest_row(row):
     for v in range(1, 3000):
         rows[v] = np.unique(rng.integers(v + 1, n, size=rng.integers(1, 300)))
     _check(*_csr(rows, n))
+
+
+def _slice_count(beg, adj, lo, hi):
+    """The counted quantity over source rows [lo, hi), rows in any order and with repeated entries."""
+    row = lambda v: adj[beg[v]:beg[v + 1]].tolist()  # noqa: E731
+    return sum(w in s for v in range(lo, hi) if beg[v + 1] - beg[v] >= 2 for s in (set(row(v)),)
+               for u in row(v) for w in row(u))
+
+
+@pytest.mark.parametrize("long_row", [129, 20])
+@pytest.mark.parametrize("schedule", [T.SCHED_LEARNED, T.SCHED_TUNED])
+def test_slices_with_duplicates_outside(long_row, schedule):
+    """A slice of increasing rows whose arcs lead to rows outside it with a repeated entry (kept arcs: the
+    slice's row is the longer; moved arcs: the repeating row is) counts with multiplicity."""
+    n = 500
+    rows = {0: np.concatenate([[5, 7, 100], np.arange(200, 200 + long_row - 3)]),
+            1: np.array([7, 100, 101]),
+            100: np.array([5, 5, 7]), 101: np.concatenate([[7, 7], np.arange(130, 330), [330] * 2])}
+    for v in range(110, 300):
+        rows[v] = np.array([v + 5, v + 9])
+    beg, adj = _csr(rows, n)
+    db, da = torch.from_numpy(beg).cuda(), torch.from_numpy(adj).cuda()
+    with T.Context() as ctx:
+        cuts = (0, 1, 2, 105, n)
+        parts = [T.count_csr(db, da, ctx=ctx, direction_split=1, schedule=schedule, row_range=(a, b))
+                 for a, b in zip(cuts[:-1], cuts[1:])]
+        assert [r.triangles for r in parts] == [_slice_count(beg, adj, a, b) for a, b in zip(cuts[:-1], cuts[1:])]
+        assert all(r.direction_split == 0 for r in parts)
+        assert sum(r.triangles for r in parts) == O.count_forward(beg, adj)
+
+
+@pytest.mark.parametrize("where", ["first", "second", "last", "none"])
+@pytest.mark.parametrize("pad", [0, 1, 2, 3])
+def test_slice_check_sees_every_row(where, pad):
+    """One repeated or descending entry anywhere outside the slice keeps it unsplit; rows that end on a
+    larger entry than the next row starts with, empty rows and one-entry rows do not."""
+    n = 3000
+    rng = np.random.default_rng(pad)
+    rows = {v: np.unique(rng.integers(0, n, size=rng.integers(0, 9))) for v in range(pad, n - pad)}
+    rows[n // 2] = np.arange(300)
+    at = {"first": min(v for v in rows if len(rows[v]) > 2), "last": max(v for v in rows if len(rows[v]) > 2)}
+    at["second"] = min(v for v in rows if len(rows[v]) > 2 and v > at["first"])
+    if where != "none":
+        rows[at[where]] = rows[at[where]][[0, 2, 1]] if where == "second" else rows[at[where]][[0, 0, 1]]
+    beg, adj = _csr(rows, n)
+    db, da = torch.from_numpy(beg).cuda(), torch.from_numpy(adj).cuda()
+    lo, hi = n // 2 - 3, n // 2 + 3
+    r = T.count_csr(db, da, direction_split=1, row_range=(lo, hi))
+    assert r.direction_split == int(where == "none") and r.triangles == _slice_count(beg, adj, lo, hi)

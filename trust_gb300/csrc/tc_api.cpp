@@ -409,6 +409,14 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     } else {
       split = sorted && split_pays(plan.w_all, plan.w_min, g.mA, g.rows);
     }
+    // the pass has checked the slice's rows; its arcs lead to rows outside it, which have to be
+    // duplicate-free as well (the whole graph's check: 0.3 ms for 170 M arcs)
+    if (split && (row_lo > 0 || (row_hi >= 0 && row_hi < g.rows))) {
+      bool increasing = false;
+      rc = rows_increasing(c, g.begA, g.adjA, g.rows, g.mA, st, &increasing);
+      if (rc) return rc;
+      split = increasing;
+    }
     if (split && bits_ok) {
       plan_wedges = plan.w_min;
       rc = prepare_bits(row_lo, row_hi < 0 ? g.rows : row_hi, plan);

@@ -169,7 +169,7 @@ int split_build(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t
 // read back like split_plan's.
 int tile_split_plan(trust_tc_ctx *c, const DevGraph3 &g, cudaStream_t st, int table_min);
 // Whether every row of a CSR is strictly increasing (so duplicate-free); synchronous.
-int rows_increasing(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t rows, cudaStream_t st,
+int rows_increasing(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t rows, int64_t m, cudaStream_t st,
                     bool *out);
 
 }  // namespace tc

@@ -277,7 +277,10 @@ __device__ __forceinline__ int tuned_class_of(int d, int warp_max, int cta_max) 
 }
 
 // Words of the scheduling pass's totals (plans[]).
-enum { PLAN_W_ALL = 0, PLAN_W_MIN = 1, PLAN_SAVED = 2, PLAN_NLONG = 3, PLAN_NPAIRS = 4, PLAN_OVERFLOW = 5 };
+enum {
+  PLAN_W_ALL = 0, PLAN_W_MIN = 1, PLAN_SAVED = 2, PLAN_NLONG = 3, PLAN_NPAIRS = 4, PLAN_OVERFLOW = 5,
+  PLAN_UNSORTED = 6  // rows_increasing's
+};
 
 // The scheduling pass, phase 1 (rows of up to TC_SCHED_FLAT entries): the split plan's probe
 // totals, the in-list count and work sum of every arc's target, the arcs the split would move
@@ -666,34 +669,49 @@ int tile_split_plan(trust_tc_ctx *c, const DevGraph3 &g, cudaStream_t st, int ta
   return TRUST_TC_OK;
 }
 
-// One warp per row: any entry not below its successor marks the CSR (flag word 1).
-__global__ void rows_increasing_kernel(const int64_t *__restrict__ beg, const int32_t *__restrict__ adj,
-                                       int64_t rows, unsigned long long *flag) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  int bad = 0;
-  for (int64_t v = warp; v < rows; v += nwarps) {
-    const long long b = tc_ld_nc(beg + v);
-    const int d = (int)(tc_ld_nc(beg + v + 1) - b);
-    for (int k = lane; k + 1 < d; k += 32) bad |= tc_ld_nc(adj + b + k) >= tc_ld_nc(adj + b + k + 1);
+// Neighbouring entries that do not increase, minus those at a row's end: zero exactly where every row is
+// strictly increasing.  One stream over the entries and one over the offsets, whatever the rows' lengths
+// (and no access depends on an offset being valid).
+__global__ void __launch_bounds__(256) rows_increasing_kernel(const int64_t *__restrict__ beg,
+                                                              const int32_t *__restrict__ adj, int64_t rows, int64_t m,
+                                                              unsigned long long *excess) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  long long n = 0;
+  for (int64_t i = tid; i + 1 < m; i += 4 * stride) {
+    int x[4], y[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int64_t k = i + r * stride;
+      x[r] = k + 1 < m ? tc_ld_nc(adj + k) : 0;
+      y[r] = k + 1 < m ? tc_ld_nc(adj + k + 1) : 1;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) n += x[r] >= y[r];
   }
-  bad = __reduce_or_sync(TC_FULL_MASK, bad);
-  if (lane == 0 && bad) atomicOr(flag, 1ull);
+  for (int64_t v = tid; v < rows; v += stride) {
+    const long long b = tc_ld_nc(beg + v), e = tc_ld_nc(beg + v + 1);
+    if (b < e && e > 0 && e < m) n -= tc_ld_nc(adj + e - 1) >= tc_ld_nc(adj + e);
+  }
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) n += __shfl_down_sync(TC_FULL_MASK, n, o);
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(excess, (unsigned long long)n);
 }
 
-int rows_increasing(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t rows, cudaStream_t st,
+int rows_increasing(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t rows, int64_t m, cudaStream_t st,
                     bool *out) {
   int rc = ensure((void **)&c->d_split_plans, &c->split_plans_cap, TC_PLAN_WORDS * sizeof(unsigned long long));
   if (rc) return rc;
-  TC_CUDA_TRY(cudaMemsetAsync(c->d_split_plans, 0, sizeof(unsigned long long), st));
-  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((rows + 7) / 8, (int64_t)c->num_sms * 8));
-  rows_increasing_kernel<<<blocks, 256, 0, st>>>(beg, adj, rows, c->d_split_plans);
+  unsigned long long *excess = c->d_split_plans + PLAN_UNSORTED;  // beside a plan's totals
+  TC_CUDA_TRY(cudaMemsetAsync(excess, 0, sizeof(unsigned long long), st));
+  const int blocks =
+      (int)std::max<int64_t>(1, std::min<int64_t>((std::max(rows, m / 4) + 255) / 256, (int64_t)c->num_sms * 16));
+  rows_increasing_kernel<<<blocks, 256, 0, st>>>(beg, adj, rows, m, excess);
   TC_NOTE_LAUNCH();
   TC_CUDA_TRY(cudaGetLastError());
-  TC_CUDA_TRY(cudaMemcpyAsync(c->h_plans, c->d_split_plans, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  TC_CUDA_TRY(cudaMemcpyAsync(c->h_plans + PLAN_UNSORTED, excess, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
   TC_CUDA_TRY(cudaStreamSynchronize(st));
-  *out = c->h_plans[0] == 0;
+  *out = c->h_plans[PLAN_UNSORTED] == 0;
   return TRUST_TC_OK;
 }
 

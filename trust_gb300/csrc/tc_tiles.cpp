@@ -120,7 +120,7 @@ static int tile_loop(trust_tc_ctx &ctx, const std::vector<Tile> &ht, bool on_dev
   auto known_increasing = [&](int id) -> int {
     if (increasing[id] >= 0) return TRUST_TC_OK;
     bool inc = false;
-    const int rc2 = rows_increasing(&ctx, dt[id].beg, dt[id].adj, ht[id].rows, (cudaStream_t)o.stream, &inc);
+    const int rc2 = rows_increasing(&ctx, dt[id].beg, dt[id].adj, ht[id].rows, ht[id].m, (cudaStream_t)o.stream, &inc);
     if (!rc2) increasing[id] = inc ? 1 : 0;
     return rc2;
   };
