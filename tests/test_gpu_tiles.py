@@ -222,3 +222,16 @@ def test_plain_schedule_tile_rows_long_in_arcs_alone(arcs, table):
         off = T.count_tiles(db, da, 2, schedule=schedule, direction_split=0)
         assert on.triangles == off.triangles == expect
         assert on.direction_split >= 1 and on.class_sizes == off.class_sizes
+
+
+@pytest.mark.parametrize("at,value", [(0, 3), (1, -7), (7, 1 << 40), (7, -(1 << 40)), (-1, 1), (-1, 1 << 33)])
+def test_folder_tiles_with_bad_offsets(tmp_path, at, value):
+    """Tiles read from a folder are checked before any access depends on their offsets."""
+    beg, adj, expect = _sorted_csr("rmat12")
+    T.partition_folder(str(tmp_path), beg.cpu().numpy(), adj.cpu().numpy(), 2)
+    b, a = T.load_folder(str(tmp_path / "partition1_0"))
+    b[at] = value
+    T.save_folder(str(tmp_path / "partition1_0"), b, a)
+    with pytest.raises(T.TrustTcError) as e:
+        T.count_partitioned(str(tmp_path), 2, direction_split=1)
+    assert e.value.status == T._lib.E_OFFSETS
