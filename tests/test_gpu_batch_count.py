@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import trust_gb300 as T
+from trust_gb300 import _lib
 from trust_gb300 import batch as B
 from oracle import oracle as O
 from tests import graphs
@@ -78,4 +79,30 @@ def test_refilled_buffers():
         adj.copy_(torch.from_numpy(a))
         counts, r = bt.run()
         assert r.triangles == int(counts.sum()) == O.count_forward(b, a)
+        bt.close()
+
+
+@pytest.mark.parametrize("made,refilled", [(100, 5000), (4096, 4097), (5000, 4097), (4097, 9000)])
+def test_refilled_with_longer_rows(made, refilled):
+    """Buffers refilled with a row longer than any the batch was made for are counted or refused, never
+    counted in part."""
+    rng = np.random.default_rng(made + refilled)
+    (beg, adj, vb), (b, a) = _union([_hub(rng, 12_000, made)]), _hub(rng, 12_000, refilled)
+    if a.size > adj.numel():  # the same number of entries: the first rows' are kept
+        b, a = np.minimum(b, adj.numel()), a[:adj.numel()]
+    else:
+        b = b.copy()
+        b[-1] = adj.numel()  # the last row takes the rest, repeated entries
+        a = np.concatenate([a, np.full(adj.numel() - a.size, 7, dtype=np.int32)])
+    expect = O.count_forward(b, a, threads=8)
+    with T.Context() as ctx:
+        bt = B.Batch(beg, adj, vb, ctx=ctx)
+        beg.copy_(torch.from_numpy(b))
+        adj.copy_(torch.from_numpy(a))
+        try:
+            counts, r = bt.run()
+            assert r.triangles == int(counts[0]) == expect
+            assert made > 4096
+        except T.TrustTcError as e:
+            assert e.status == _lib.E_DEVICE and refilled > made
         bt.close()
