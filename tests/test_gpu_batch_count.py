@@ -106,3 +106,25 @@ def test_refilled_with_longer_rows(made, refilled):
         except T.TrustTcError as e:
             assert e.status == _lib.E_DEVICE and refilled > made
         bt.close()
+
+
+@pytest.mark.parametrize("which,at,value,status", [("adj", 0, -1, _lib.E_IDS), ("adj", -1, 1 << 30, _lib.E_IDS),
+                                                   ("beg", 0, 2, _lib.E_OFFSETS), ("beg", 300, -5, _lib.E_OFFSETS),
+                                                   ("beg", 300, 1 << 40, _lib.E_OFFSETS), ("beg", -1, 1, _lib.E_OFFSETS)])
+def test_refilled_with_invalid_input(which, at, value, status):
+    """Refilled buffers are validated by every run before a row or entry of theirs is indexed."""
+    rng = np.random.default_rng(7)
+    cs = [_er(rng, 400, 30), _hub(rng, 6000, 5000), _er(rng, 3000, 6)]
+    beg, adj, vb = _union(cs)
+    expect = [O.count_forward(b, a) for b, a in cs]
+    with T.Context() as ctx:
+        bt = B.Batch(beg, adj, vb, ctx=ctx)
+        x = beg if which == "beg" else adj
+        keep = x[at].clone()
+        x[at] = value
+        with pytest.raises(T.TrustTcError) as e:
+            bt.run()
+        assert e.value.status == status
+        x[at] = keep
+        assert list(bt.run()[0]) == expect
+        bt.close()

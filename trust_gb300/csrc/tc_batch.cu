@@ -205,6 +205,7 @@ int batch_enqueue(trust_tc_batch *b, cudaStream_t st, bool timed) {
   a.adj = b->adj;
   a.lists = b->d_lists;
   a.ctl = b->d_ctl + TC_BATCH_CLASSES;  // the combined lists of every size class
+  a.checked = b->d_ctl;
   a.graph_of = b->d_graph_of;
   a.graph_vbeg = b->d_vbeg;
   a.graph_counts = b->d_counts;

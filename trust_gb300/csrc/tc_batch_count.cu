@@ -491,6 +491,8 @@ __global__ void __launch_bounds__(MAXT, MINB) batch_count_kernel(BatchCountArgs 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   unsigned char *wl = reinterpret_cast<unsigned char *>(smem) + p.table_bytes + warp * WL_BYTES;
+  // The host reads the status after the whole job: rows and entries are indexed only if they are valid.
+  if (p.checked->status) return;
   if (threadIdx.x == 0) bs.count = bs.wedges = 0;
   unsigned long long wedges = 0;
   GraphAcc acc{-1, 0, 0};
