@@ -88,3 +88,26 @@ def test_invalid_input(ctx):
             T.count_csr(*_dev(b, adj), ctx=ctx)
         assert e.value.status == _lib.E_OFFSETS
         assert T.count_csr(*_dev(beg, adj), ctx=ctx).triangles == expect
+
+
+def test_first_call_on_a_capturing_stream():
+    """A call cannot be captured (it synchronises): it fails, and the context's next call counts."""
+    beg, adj = O.build_csr(graphs.complete(60)[0], 60)
+    db, da = _dev(beg, adj)
+    dirty = [torch.full((64,), -1, dtype=torch.int64, device="cuda") for _ in range(64)]  # no zeroed memory by chance
+    del dirty
+    torch.cuda.empty_cache()
+    with T.Context() as c:
+        s = torch.cuda.Stream()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(s):
+            g.capture_begin(capture_error_mode="relaxed")
+            with pytest.raises(T.TrustTcError) as e:
+                T.count_csr(db, da, ctx=c, stream=s.cuda_stream)
+            try:
+                g.capture_end()
+            except RuntimeError:  # the capture is invalid
+                pass
+        assert e.value.status == _lib.E_CUDA
+        for _ in range(2):
+            assert T.count_csr(db, da, ctx=c).triangles == graphs.complete(60)[1]

@@ -54,13 +54,17 @@ int ctx_init(trust_tc_ctx *c, int device) {
   TC_CUDA_TRY(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device));
   TC_CUDA_TRY(cudaDeviceGetAttribute(&c->max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   TC_CUDA_TRY(cudaDeviceGetAttribute(&c->clock_khz, cudaDevAttrClockRate, device));
-  TC_CUDA_TRY(cudaMalloc(&c->d_ctl, sizeof(TcControl)));
+  TC_CUDA_TRY(cudaMalloc(&c->d_ctl, 2 * sizeof(TcControl)));
+  c->d_small = c->d_ctl + 1;
   TC_CUDA_TRY(cudaMallocHost(&c->h_ctl, sizeof(TcControl)));
   TC_CUDA_TRY(cudaMallocHost(&c->h_plans, TC_PLAN_WORDS * sizeof(unsigned long long)));
   for (auto &ev : c->ev) TC_CUDA_TRY(cudaEventCreate(&ev));
   for (auto &ev : c->ev_split) TC_CUDA_TRY(cudaEventCreate(&ev));
   for (auto &sl : c->staged) TC_CUDA_TRY(cudaEventCreateWithFlags(&sl.ready, cudaEventDisableTiming));
   TC_CUDA_TRY(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
+  // zeroed here, not by the first call: the first call's stream may be capturing, and would only record it
+  TC_CUDA_TRY(cudaMemsetAsync(c->d_small, 0, sizeof(TcControl), c->copy_stream));
+  TC_CUDA_TRY(cudaStreamSynchronize(c->copy_stream));
   return TRUST_TC_OK;
 }
 
@@ -109,7 +113,6 @@ void ctx_release(trust_tc_ctx *c) {
   cudaFree(c->d_split_cbeg);
   cudaFree(c->d_split_rowmap);
   cudaFree(c->d_split_adj);
-  cudaFree(c->d_small);
   cudaFree(c->d_bits_cols);
   cudaFree(c->d_bits_ent);
   cudaFree(c->d_bits_desc);

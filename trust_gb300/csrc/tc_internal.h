@@ -55,7 +55,7 @@ struct trust_tc_ctx {
   size_t split_rowmap_cap = 0;
   int32_t *d_split_adj = nullptr;
   size_t split_adj_cap = 0;
-  TcControl *d_small = nullptr;  // accumulators of the one-launch path, zero between calls
+  TcControl *d_small = nullptr;  // behind d_ctl: accumulators of the one-launch path, zero between calls
   unsigned *d_bits_cols = nullptr;  // block-bitmap path: column popularity and ranks, counters, row lists
   size_t bits_cols_cap = 0;
   unsigned *d_bits_ent = nullptr;  // every row as block entries, then tail ids

@@ -199,10 +199,6 @@ bool small_graph(int64_t n, int64_t m) { return n >= 1 && n <= SMALL_MAX_IDS && 
 
 int small_count(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, int64_t row_lo,
                 int64_t row_hi, int check_ids, int warp_max, int cta_max, cudaStream_t st) {
-  if (!c->d_small) {
-    TC_CUDA_TRY(cudaMalloc((void **)&c->d_small, sizeof(TcControl)));
-    TC_CUDA_TRY(cudaMemsetAsync(c->d_small, 0, sizeof(TcControl), st));
-  }
   SmallArgs a;
   a.beg = beg;
   a.adj = adj;
