@@ -111,3 +111,34 @@ def test_first_call_on_a_capturing_stream():
         assert e.value.status == _lib.E_CUDA
         for _ in range(2):
             assert T.count_csr(db, da, ctx=c).triangles == graphs.complete(60)[1]
+
+
+def test_callers_streams_and_contexts_at_once():
+    """Non-blocking streams and several contexts at a time, one host thread each."""
+    import threading
+    rng = np.random.default_rng(3)
+    beg, adj = graphs.random_csr(rng, 500, 90)
+    expect = O.count_forward(beg, adj)
+    pairs = T.gen_rmat(15, 24, 0.7, 0.125, 0.125, seed=3)
+    big = T.build_csr(pairs, 1 << 15)
+    whole = O.count_forward(*(x.cpu().numpy() for x in big), threads=8)
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(k):
+        s = torch.cuda.Stream()
+        db, da = _dev(beg, adj)
+        torch.cuda.synchronize()
+        with T.Context() as c:
+            for _ in range(20):
+                r = T.count_csr(db, da, ctx=c, stream=s.cuda_stream)
+                b = T.count_csr(*big, ctx=c, stream=s.cuda_stream, direction_split=1)
+                if r.triangles != expect or b.triangles != whole or b.direction_split != 1:
+                    wrong.append((k, r, b))
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not wrong
