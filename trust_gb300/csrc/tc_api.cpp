@@ -35,6 +35,7 @@ void note_launch(uint64_t k) { g_kernel_launches.fetch_add(k, std::memory_order_
 int cuda_status(cudaError_t e) {
   if (e == cudaSuccess) return TRUST_TC_OK;
   snprintf(g_cuda_err, sizeof g_cuda_err, "%s (%s)", cudaGetErrorString(e), cudaGetErrorName(e));
+  cudaGetLastError();  // reported here: the check after the next launch is for that launch alone
   if (e == cudaErrorMemoryAllocation) return TRUST_TC_E_NOMEM;
   if (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver) return TRUST_TC_E_NO_DEVICE;
   return TRUST_TC_E_CUDA;
@@ -239,10 +240,61 @@ static bool split_pays(unsigned long long w_all, unsigned long long w_min, int64
 static int split_second_pass(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bool same,
                              int64_t max_out_degree, trust_tc_result *rb, float *t_build);
 
-// The device-side counting call over three CSRs (A = tables, B = arcs, C = probe lists).
-// `check_*` select which CSRs get an id-range check on the device.
-int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bool check_ids,
-                 trust_tc_result *r) {
+// Free the scratch of the scheduling pass and of the split (both grow with the arcs).
+static void release_split_scratch(trust_tc_ctx *c) {
+  if (c->sub) {
+    ctx_release(c->sub);
+    delete c->sub;
+    c->sub = nullptr;
+  }
+  auto drop = [](auto *&p, size_t &cap) {
+    cudaFree(p);
+    p = nullptr;
+    cap = 0;
+  };
+  drop(c->d_split_pairs, c->split_pairs_cap);
+  drop(c->d_split_place, c->split_place_cap);
+  drop(c->d_split_beg, c->split_beg_cap);
+  drop(c->d_split_cbase, c->split_cbase_cap);
+  drop(c->d_split_cbeg, c->split_cbeg_cap);
+  drop(c->d_split_rowmap, c->split_rowmap_cap);
+  drop(c->d_split_adj, c->split_adj_cap);
+  drop(c->d_split_cnt, c->split_cnt_cap);
+  drop(c->d_split_wsum, c->split_wsum_cap);
+  drop(c->d_sched_long, c->sched_long_cap);
+  drop(c->d_deg, c->deg_cap);
+  drop(c->d_dec, c->dec_cap);
+  drop(c->d_pred, c->pred_cap);
+  drop(c->d_sort, c->sort_cap);
+  drop(c->d_bits_cols, c->bits_cols_cap);
+  drop(c->d_bits_ent, c->bits_ent_cap);
+  drop(c->d_bits_desc, c->bits_desc_cap);
+  drop(c->d_bits_units, c->bits_units_cap);
+}
+
+static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bool check_ids,
+                                trust_tc_result *r, bool *planned);
+
+// The device-side counting call.  Where the scheduling pass or the split finds no memory (14 bytes per
+// arc, and 9 more for the block bitmaps), its scratch is given back and the arcs are counted unsplit in
+// the tuned classes.  The two hash passes are not tried in between: they take 16 bytes per arc more.
+int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bool check_ids, trust_tc_result *r) {
+  bool planned = false;
+  int rc = count_device_planned(c, g, o, check_ids, r, &planned);
+  if (rc != TRUST_TC_E_NOMEM || !planned) return rc;
+  TC_CUDA_TRY(cudaStreamSynchronize((cudaStream_t)o.stream));
+  if (c->sub_stream) TC_CUDA_TRY(cudaStreamSynchronize(c->sub_stream));
+  release_split_scratch(c);
+  trust_tc_opts unsplit = o;
+  unsplit.direction_split = 0;
+  if (unsplit.schedule == TRUST_TC_SCHED_LEARNED) unsplit.schedule = TRUST_TC_SCHED_TUNED;
+  return count_device_planned(c, g, unsplit, check_ids, r, &planned);
+}
+
+// The call over three CSRs (A = tables, B = arcs, C = probe lists), ids range-checked with check_ids.
+// *planned: the call went as far as the scheduling pass.
+static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bool check_ids,
+                                trust_tc_result *r, bool *planned) {
   cudaStream_t st = (cudaStream_t)o.stream;
   const bool same = g.begA == g.begB && g.begB == g.begC && g.adjA == g.adjB && g.adjB == g.adjC;
   LaunchCfg cfg;
@@ -371,6 +423,7 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     return bits_prepare(c, g, lo, hi, plan, h.max_out_degree, c->sub_stream, &bits);
   };
   if (consider) {
+    *planned = true;
     const float *d_model = nullptr;
     if (learned) {
       rc = load_model(c, o.model, &d_model);
@@ -423,9 +476,8 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     if (split && bits_ok) {
       plan_wedges = plan.w_min;
       rc = prepare_bits(row_lo, row_hi < 0 ? g.rows : row_hi, plan);
-      if (rc == TRUST_TC_E_NOMEM) split = 0;  // no room for the blocks (allocated first): count unsplit
-      else if (rc) return rc;
-      use_bits = rc == TRUST_TC_OK;
+      if (rc) return rc;
+      use_bits = true;
     }
   }
   // a tile job (three CSRs, duplicate-free tables and probe rows): the same split, decided by the
@@ -435,6 +487,7 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
                           (o.direction_split < 0 && o.schedule == TRUST_TC_SCHED_LEARNED &&
                            h.max_out_degree >= 64 && g.mB >= TC_LEARNED_MIN_ARCS));
   if (consider3) {
+    *planned = true;
     rc = tile_split_plan(c, g, st, bits_ok ? BITS_TABLE_MIN : 0);
     if (rc) return rc;
     TC_CUDA_TRY(cudaStreamSynchronize(st));
@@ -445,9 +498,8 @@ int count_device(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bo
     if (split && bits_ok) {
       plan_wedges = plan.w_min;
       rc = prepare_bits(0, g.rows, plan);
-      if (rc == TRUST_TC_E_NOMEM) split = 0;  // as for one graph
-      else if (rc) return rc;
-      use_bits = rc == TRUST_TC_OK;
+      if (rc) return rc;
+      use_bits = true;
     }
   }
   // the fused pass's lists stand unless the learned decisions re-classified the rows
