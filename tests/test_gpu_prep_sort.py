@@ -62,3 +62,28 @@ def test_unaligned_pairs_and_invalid_ids():
 def test_no_pairs():
     beg, adj = T.build_csr(torch.empty((0, 2), dtype=torch.int32, device="cuda"), 7)
     assert beg.tolist() == [0] and adj.numel() == 0
+
+
+@pytest.mark.parametrize("npairs", [1, 2, 5000])
+@pytest.mark.parametrize("over", [-1, 0, 1, 100_000, (1 << 26)])
+def test_ids_far_apart(npairs, over):
+    """Around as many ids as the pairs have ends (out-degrees by id, then by compacted id), renumbered and in
+    batches, where the order is kept."""
+    ids = 2 * npairs + over
+    rng = np.random.default_rng(ids)
+    p = rng.integers(0, ids, size=(npairs, 2)).astype(np.int32)
+    p[-1] = [0, ids - 1]
+    eb, ea = O.build_csr(p, ids)
+    gb, ga = T.build_csr(torch.from_numpy(p).cuda(), ids)
+    np.testing.assert_array_equal(gb.cpu().numpy(), eb)
+    np.testing.assert_array_equal(ga.cpu().numpy(), ea)
+    from trust_gb300 import batch as B
+    bb, ba, gv = B.build_batch(torch.from_numpy(p).cuda(), np.array([0, ids // 3, ids], dtype=np.int64))
+    present = np.unique(p[p[:, 0] != p[:, 1]])
+    e = np.unique(np.sort(np.searchsorted(present, p[p[:, 0] != p[:, 1]]), axis=1), axis=0)
+    deg = np.bincount(e.ravel(), minlength=present.size)
+    e[deg[e[:, 0]] > deg[e[:, 1]]] = e[deg[e[:, 0]] > deg[e[:, 1]]][:, ::-1]
+    e = e[np.lexsort((e[:, 1], e[:, 0]))]
+    np.testing.assert_array_equal(ba.cpu().numpy(), e[:, 1])
+    np.testing.assert_array_equal(np.diff(bb.cpu().numpy()), np.bincount(e[:, 0], minlength=present.size))
+    assert list(gv) == [0, int(np.searchsorted(present, ids // 3)), present.size]
