@@ -196,7 +196,7 @@ int batch_enqueue(trust_tc_batch *b, cudaStream_t st, bool timed) {
   if ((rc = launch_batch_classify(0, b->beg, b->n, b->d_graph_of, b->d_graph_sc, th, b->d_ctl, b->d_lists, num_sms,
                                   st)))
     return rc;
-  if ((rc = launch_batch_offsets(b->d_ctl, TC_BATCH_CLASSES, st))) return rc;
+  if ((rc = launch_batch_offsets(b->d_ctl, TC_BATCH_CLASSES, b->huge_blocks, st))) return rc;
   if ((rc = launch_batch_classify(1, b->beg, b->n, b->d_graph_of, b->d_graph_sc, th, b->d_ctl, b->d_lists, num_sms,
                                   st)))
     return rc;
@@ -205,7 +205,6 @@ int batch_enqueue(trust_tc_batch *b, cudaStream_t st, bool timed) {
   a.adj = b->adj;
   a.lists = b->d_lists;
   a.ctl = b->d_ctl + TC_BATCH_CLASSES;  // the combined lists of every size class
-  a.checked = b->d_ctl;
   a.graph_of = b->d_graph_of;
   a.graph_vbeg = b->d_vbeg;
   a.graph_counts = b->d_counts;

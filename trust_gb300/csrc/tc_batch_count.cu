@@ -491,8 +491,6 @@ __global__ void __launch_bounds__(MAXT, MINB) batch_count_kernel(BatchCountArgs 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   unsigned char *wl = reinterpret_cast<unsigned char *>(smem) + p.table_bytes + warp * WL_BYTES;
-  // The host reads the status after the whole job: rows and entries are indexed only if they are valid.
-  if (p.checked->status) return;
   if (threadIdx.x == 0) bs.count = bs.wedges = 0;
   unsigned long long wedges = 0;
   GraphAcc acc{-1, 0, 0};
@@ -501,11 +499,7 @@ __global__ void __launch_bounds__(MAXT, MINB) batch_count_kernel(BatchCountArgs 
   for (int c = TC_CLASS_HUGE; c >= TC_CLASS_CTA; --c) {
     const int n_items = p.ctl->class_count[c];
     if (n_items == 0) continue;
-    if (c == TC_CLASS_HUGE && (int)blockIdx.x >= p.huge_blocks) {
-      // (buffers refilled with such rows, the batch made for none)
-      if (p.huge_blocks == 0 && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&p.ctl->status, TC_DEV_TABLE_FULL);
-      continue;
-    }
+    if (c == TC_CLASS_HUGE && (int)blockIdx.x >= p.huge_blocks) continue;
     const int *list = class_list(p, c);
     int *tab = (c == TC_CLASS_HUGE) ? p.huge_tables + (size_t)blockIdx.x * ((size_t)1 << p.huge_log2) : smem;
     for (;;) {

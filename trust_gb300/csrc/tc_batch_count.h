@@ -9,7 +9,6 @@ struct BatchCountArgs {
   const int32_t *adj;
   const int *lists;          // every degree class's rows, at ctl->class_off
   TcControl *ctl;            // the combined block: list sizes and offsets, queue heads, count
-  const TcControl *checked;  // the block whose status holds the union's validation
   const int *graph_of;       // graph of every row
   const int64_t *graph_vbeg; // graph g's ids: [graph_vbeg[g], graph_vbeg[g + 1])
   unsigned long long *graph_counts;

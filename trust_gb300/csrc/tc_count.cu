@@ -656,9 +656,13 @@ __global__ void batch_class_kernel(const int64_t *__restrict__ beg, int64_t rows
 
 // List offsets of every (size class, degree class), degree class major: each degree class's rows
 // of all size classes are contiguous, so ctl[nsc] (the combined block) describes them as one list
-// per degree class, drained by one persistent counting kernel.
-__global__ void batch_offsets_kernel(TcControl *ctl, int nsc) {
+// per degree class, drained by one persistent counting kernel.  The host reads the status after the
+// whole job, so what must not be counted is decided here (in the counting kernel the same test costs 1 % of a
+// run of 4096 graphs): nothing of invalid input, and no rows above the CTA class where the batch was made for
+// none (buffers refilled since) and has no tables for them.
+__global__ void batch_offsets_kernel(TcControl *ctl, int nsc, int huge_blocks) {
   if (blockIdx.x != 0 || threadIdx.x != 0) return;
+  const bool valid = ctl[0].status == 0;
   int run = 0;
   for (int c = 0; c < TC_NUM_CLASSES; ++c) {
     ctl[nsc].class_off[c] = run;
@@ -670,8 +674,9 @@ __global__ void batch_offsets_kernel(TcControl *ctl, int nsc) {
         all += ctl[s].class_count[c];
       }
     }
-    ctl[nsc].class_count[c] = all;
+    ctl[nsc].class_count[c] = valid ? all : 0;
   }
+  if (ctl[nsc].class_count[TC_CLASS_HUGE] > 0 && huge_blocks == 0) ctl[nsc].status |= TC_DEV_TABLE_FULL;
 }
 
 int launch_batch_classify(int pass, const int64_t *beg, int64_t rows, const int *graph_of,
@@ -687,8 +692,8 @@ int launch_batch_classify(int pass, const int64_t *beg, int64_t rows, const int 
   return TRUST_TC_OK;
 }
 
-int launch_batch_offsets(TcControl *ctl, int nsc, cudaStream_t st) {
-  batch_offsets_kernel<<<1, 32, 0, st>>>(ctl, nsc);
+int launch_batch_offsets(TcControl *ctl, int nsc, int huge_blocks, cudaStream_t st) {
+  batch_offsets_kernel<<<1, 32, 0, st>>>(ctl, nsc, huge_blocks);
   TC_NOTE_LAUNCH();
   TC_CUDA_TRY(cudaGetLastError());
   return TRUST_TC_OK;

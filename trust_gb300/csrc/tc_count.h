@@ -72,7 +72,7 @@ struct BatchThresholds {
 int launch_batch_classify(int pass, const int64_t *beg, int64_t rows, const int *graph_of,
                           const unsigned char *graph_sc, const BatchThresholds &th, TcControl *ctl, int *lists,
                           int num_sms, cudaStream_t st);
-int launch_batch_offsets(TcControl *ctl, int nsc, cudaStream_t st);
+int launch_batch_offsets(TcControl *ctl, int nsc, int huge_blocks, cudaStream_t st);
 // Hub rows (huge class, out-degree <= a.hub_max_degree) on clusters of 2^log2C CTAs of 512
 // threads; tables up to 2^max_log2 slots, 2^(max_log2 - log2C) per CTA in shared memory.
 int launch_hub(bool same, const CountArgs &a, int max_log2, int log2C, int clusters, cudaStream_t st);
