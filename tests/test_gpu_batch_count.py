@@ -128,3 +128,14 @@ def test_refilled_with_invalid_input(which, at, value, status):
         x[at] = keep
         assert list(bt.run()[0]) == expect
         bt.close()
+
+
+@pytest.mark.parametrize("n", [55_423, 55_424, 55_425, 120_000])
+@pytest.mark.parametrize("share", [0, 1, 2])
+def test_graphs_around_the_bitmap_bound(n, share):
+    """Graphs whose ids just fit the words of a warp, just do not, or by far do not, alone and beside as many
+    vertices, or more, in graphs that do (bitmaps only where those hold half of the vertices)."""
+    rng = np.random.default_rng(n + share)
+    cs = [_er(rng, n, d) for d in (6, 30, 64)] + [_hub(rng, n, 4500)]
+    cs += [_er(rng, 40_000, 30) for _ in range(share * len(cs) * n // 40_000)] + [_er(rng, 50, 49), _hub(rng, 8000, 70)]
+    _check(cs, ((256, 128, 8), (1024, 64, 4)))

@@ -29,9 +29,8 @@ namespace {
 
 // size classes by vertex count: [0, 512), [512, 4096), [4096, 32768), [32768, ...)
 constexpr int64_t SC_LIMIT[TC_BATCH_CLASSES - 1] = {512, 4096, 32768};
-// Bitmap words per warp: graphs of up to 50,176 vertices, and still four CTAs of eight warps per SM
-// (4096 graphs of up to 50,000, ms per run: 512 words 17.1, 1024 15.4, 1568 13.9).
-constexpr int BITMAP_WORDS = 1568;
+constexpr int GROUP_KEYS = 32;   // words of a warp's region that hold the group classes' keys
+constexpr int HASH_WORDS = 256;  // without bitmaps: the group classes' hash table
 constexpr int CTA_MAX = 4096;  // CTA-class bound of every size class (hub rows above it spill)
 
 int size_class_of(int64_t nv) {
@@ -87,11 +86,17 @@ struct trust_tc_batch {
   const int32_t *adj = nullptr;
   int64_t n = 0, m = 0, G = 0;
   int64_t graphs[TC_BATCH_CLASSES] = {}, vertices[TC_BATCH_CLASSES] = {};
-  int64_t max_vertices[TC_BATCH_CLASSES] = {};  // of one graph
+  // Bitmaps over a graph's ids: the words per warp that still leave four CTAs of eight warps per SM (4096
+  // graphs of up to 50,000, ms per run: 512 words 17.1, 1024 15.4, 1568 13.9; 200 graphs of 54,000 that fit
+  // since the device's memory sets the bound 6.4 -> 5.6), and by size class the largest graph that fits them and
+  // the vertices of all that fit.
+  int bitmap_words = 0;
+  int64_t fit_ids[TC_BATCH_CLASSES] = {}, fit_vertices[TC_BATCH_CLASSES] = {};
   int maxdeg[TC_BATCH_CLASSES] = {};
   trust_tc_batch_class cfg[TC_BATCH_CLASSES];
   // the resolved counting launch (one for every size class)
   int threads = 256, chunk = 8, blocks = 0, warp_words = 0;
+  bool bitmaps = true;
   size_t smem = 0;
   int64_t *d_vbeg = nullptr;
   int *d_graph_of = nullptr;
@@ -159,22 +164,29 @@ int batch_prepare(trust_tc_batch *b) {
       dcta = std::max(dcta, std::min(b->maxdeg[s], CTA_MAX));
     }
   }
-  // the bitmap of a graph's ids where that takes at most BITMAP_WORDS words per warp, and the 32 keys
-  // of the group classes
-  int64_t ids = 0;
+  // a bitmap over the ids of the largest graph that fits one, unless the graphs too large for it hold most of
+  // the vertices: those are better served by hash tables and the L1 that the words would take (one graph of 2 M
+  // vertices 0.67 -> 0.46 ms, with 2000 of 100 beside it 0.73 -> 0.52)
+  int64_t ids = 0, fit = 0, all = 0;
   for (int s = 0; s < TC_BATCH_CLASSES; ++s)
-    if (b->graphs[s] && b->maxdeg[s] > 8) ids = std::max(ids, b->max_vertices[s]);
-  b->warp_words = std::max(std::max(slots, 128), (int)std::min<int64_t>((ids + 127) / 128 * 4, BITMAP_WORDS) + 32);
+    if (b->graphs[s] && b->maxdeg[s] > 8) {
+      ids = std::max(ids, b->fit_ids[s]);
+      fit += b->fit_vertices[s];
+      all += b->vertices[s];
+    }
+  b->bitmaps = 2 * fit >= all;
+  b->warp_words = std::max(std::max(slots, b->bitmaps ? 128 : HASH_WORDS),
+                           b->bitmaps ? (int)((ids + 127) / 128 * 4) + GROUP_KEYS : 0);
   size_t sm = (size_t)4 * b->warp_words * warps;
   if (sm > (size_t)b->ctx->max_smem_optin) {  // many warps: what the hash tables need
-    b->warp_words = std::max(slots, 128);
+    b->warp_words = std::max(slots, b->bitmaps ? 128 : HASH_WORDS);
     sm = (size_t)4 * b->warp_words * warps;
   }
   if (cta) sm = std::max(sm, (size_t)4 << std::max(ceil_log2(2 * (int64_t)dcta), 6));
   if (sm > (size_t)b->ctx->max_smem_optin) return TRUST_TC_E_ARG;
   b->smem = sm;
   int per_sm = 0;
-  int rc = batch_count_occupancy(b->threads, sm, &per_sm);
+  int rc = batch_count_occupancy(b->threads, b->bitmaps, sm, &per_sm);
   if (rc) return rc;
   if (per_sm < 1) return TRUST_TC_E_ARG;
   b->blocks = num_sms * per_sm;
@@ -215,7 +227,7 @@ int batch_enqueue(trust_tc_batch *b, cudaStream_t st, bool timed) {
   a.table_bytes = (int)b->smem;
   a.chunk = b->chunk;
   if (timed) TC_CUDA_TRY(cudaEventRecord(b->ev[2], st));
-  if ((rc = launch_batch_count(a, b->blocks, b->threads, st))) return rc;
+  if ((rc = launch_batch_count(a, b->blocks, b->threads, b->bitmaps, st))) return rc;
   if (timed) TC_CUDA_TRY(cudaEventRecord(b->ev[3], st));
   TC_CUDA_TRY(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(TcControl) * NCTL, cudaMemcpyDeviceToHost, st));
   TC_CUDA_TRY(cudaMemcpyAsync(b->h_counts, b->d_counts, sizeof(unsigned long long) * (size_t)b->G,
@@ -282,22 +294,27 @@ int trust_tc_batch_create(trust_tc_ctx *ctx, const int64_t *d_begin, const int32
   b->n = n;
   b->m = m;
   b->G = num_graphs;
+  auto fail = [&](int rc) {
+    batch_release(b);
+    delete b;
+    return rc;
+  };
+  int rc = batch_count_warp_words(&b->bitmap_words);
+  if (rc) return fail(rc);
+  b->bitmap_words -= GROUP_KEYS;
   std::vector<unsigned char> sc((size_t)num_graphs);
   for (int64_t g = 0; g < num_graphs; ++g) {
     const int64_t nv = graph_vbeg[g + 1] - graph_vbeg[g];
     sc[(size_t)g] = (unsigned char)size_class_of(nv);
     b->graphs[sc[(size_t)g]] += 1;
     b->vertices[sc[(size_t)g]] += nv;
-    b->max_vertices[sc[(size_t)g]] = std::max(b->max_vertices[sc[(size_t)g]], nv);
+    if (nv <= 32 * (int64_t)b->bitmap_words) {
+      b->fit_ids[sc[(size_t)g]] = std::max(b->fit_ids[sc[(size_t)g]], nv);
+      b->fit_vertices[sc[(size_t)g]] += nv;
+    }
   }
   for (auto &c : b->cfg) c = trust_tc_batch_class{256, 128, 8};
-  auto fail = [&](int rc) {
-    batch_release(b);
-    delete b;
-    return rc;
-  };
   auto cu = [&](cudaError_t e) { return e == cudaSuccess ? TRUST_TC_OK : cuda_status(e); };
-  int rc = TRUST_TC_OK;
   if ((rc = cu(cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking)))) return fail(rc);
   for (auto &e : b->ev)
     if ((rc = cu(cudaEventCreate(&e)))) return fail(rc);

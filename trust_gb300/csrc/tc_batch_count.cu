@@ -374,12 +374,25 @@ __device__ __forceinline__ void warp_vertex(const BatchCountArgs &p, int v, int 
 }
 
 // The warp's 32/G vertices (lane: its row entry u or -1, that entry's row (s, dd)).  G >= 16: the
-// filter words are zero on entry and on return; the region's last 32 words hold the keys.
-template <int G>
+// filter words are zero on entry and on return; the region's last 32 words hold the keys.  Without
+// BITMAPS (the graphs' ids do not fit the words) 16-entry rows are walked as shorter ones are, and 32-entry rows
+// take a hash table, left as it is: filters there let entries pass that cost a search of the keys (one graph
+// of 2 M vertices and 16 M arcs 0.59 -> 0.46 ms, 200 of 60,000 and 1.8 M arcs 7.1 -> 6.8).
+constexpr int HASH32_LOG2 = 8;
+template <int G, bool BITMAPS>
 __device__ __forceinline__ void group_vertices(const BatchCountArgs &p, int u, int s, int dd, int *wtab, IdSpace sp,
                                                unsigned char *wl, unsigned long long &hits) {
-  if constexpr (G <= 8) {
+  if constexpr (G <= 8 || (G == 16 && !BITMAPS)) {
     probe_short<G>(p.adj, s, dd, u, hits);
+  } else if constexpr (!BITMAPS) {  // one vertex of up to 32 entries
+    const int lane = threadIdx.x & 31;
+    int4 *slots = reinterpret_cast<int4 *>(wtab);
+    slots[lane] = slots[lane + 32] = make_int4(-1, -1, -1, -1);
+    __syncwarp();
+    if (u >= 0) set_insert(wtab, HASH32_LOG2, u);
+    __syncwarp();
+    probe_chunks(p.adj, s, dd, wl, HashSet{wtab, HASH32_LOG2}, hits);
+    __syncwarp();
   } else {
     const int lane = threadIdx.x & 31;
     unsigned *words = reinterpret_cast<unsigned *>(wtab);
@@ -413,7 +426,7 @@ struct GroupStage {
 // Drain one group class.  Each warp claims `chunk` steps of 32/G vertices.  Loads run three steps
 // ahead: while step t is probed, step t+1's target rows, step t+2's row entries and step t+3's row
 // bounds are in flight.
-template <int G>
+template <int G, bool BITMAPS>
 __device__ void drain_groups(const BatchCountArgs &p, int c, int *warp_tab, unsigned char *wl, GraphAcc &acc,
                              unsigned long long &wedges) {
   constexpr int GPW = 32 / G;
@@ -473,7 +486,7 @@ __device__ void drain_groups(const BatchCountArgs &p, int c, int *warp_tab, unsi
         const int dd = mine ? s0.dd : 0;
         unsigned long long hits = 0;
         wedges += (unsigned)dd;
-        group_vertices<G>(p, mine ? s0.u : -1, s0.s, dd, warp_tab, sp, wl, hits);
+        group_vertices<G, BITMAPS>(p, mine ? s0.u : -1, s0.s, dd, warp_tab, sp, wl, hits);
         acc_take(p, acc, gx, hits);
         pending &= ~__ballot_sync(TC_FULL_MASK, mine);
       }
@@ -484,7 +497,7 @@ __device__ void drain_groups(const BatchCountArgs &p, int c, int *warp_tab, unsi
   }
 }
 
-template <int MAXT, int MINB>
+template <int MAXT, int MINB, bool BITMAPS>
 __global__ void __launch_bounds__(MAXT, MINB) batch_count_kernel(BatchCountArgs p) {
   extern __shared__ int smem[];
   __shared__ BlockShared bs;
@@ -538,10 +551,10 @@ __global__ void __launch_bounds__(MAXT, MINB) batch_count_kernel(BatchCountArgs 
       }
     }
   }
-  drain_groups<32>(p, TC_CLASS_G32, warp_tab, wl, acc, wedges);
-  drain_groups<16>(p, TC_CLASS_G16, warp_tab, wl, acc, wedges);
-  drain_groups<8>(p, TC_CLASS_G8, warp_tab, wl, acc, wedges);
-  drain_groups<4>(p, TC_CLASS_G4, warp_tab, wl, acc, wedges);
+  drain_groups<32, BITMAPS>(p, TC_CLASS_G32, warp_tab, wl, acc, wedges);
+  drain_groups<16, BITMAPS>(p, TC_CLASS_G16, warp_tab, wl, acc, wedges);
+  drain_groups<8, BITMAPS>(p, TC_CLASS_G8, warp_tab, wl, acc, wedges);
+  drain_groups<4, BITMAPS>(p, TC_CLASS_G4, warp_tab, wl, acc, wedges);
   acc_flush(p, acc);
 
   unsigned long long hits = acc.total;
@@ -559,39 +572,64 @@ __global__ void __launch_bounds__(MAXT, MINB) batch_count_kernel(BatchCountArgs 
 
 // Two register budgets: up to 1024 threads per CTA, or <= 256 with four CTAs resident per SM (with
 // five the kernel spills: 17.7 against 15.4 ms per run of 4096 graphs).
-const void *kernel_for(int threads) {
-  return threads <= 256 ? (const void *)batch_count_kernel<256, 4> : (const void *)batch_count_kernel<1024, 1>;
+const void *kernel_for(int threads, bool bitmaps) {
+  if (threads <= 256)
+    return bitmaps ? (const void *)batch_count_kernel<256, 4, true> : (const void *)batch_count_kernel<256, 4, false>;
+  return bitmaps ? (const void *)batch_count_kernel<1024, 1, true> : (const void *)batch_count_kernel<1024, 1, false>;
 }
 
 size_t smem_for(size_t table_bytes, int threads) { return table_bytes + (size_t)WL_BYTES * (threads / 32); }
 
 }  // namespace
 
-int batch_count_occupancy(int threads, size_t table_bytes, int *blocks_per_sm) {
-  const void *fn = kernel_for(threads);
-  const int smem = (int)smem_for(table_bytes, threads);
-  TC_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+static int shared_limits(const void *fn, int *per_sm, int *reserved, int *most) {
   int dev = 0, optin = 0;
   TC_CUDA_TRY(cudaGetDevice(&dev));
+  TC_CUDA_TRY(cudaDeviceGetAttribute(per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+  TC_CUDA_TRY(cudaDeviceGetAttribute(reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
   TC_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   cudaFuncAttributes at;
   TC_CUDA_TRY(cudaFuncGetAttributes(&at, fn));
-  const int most = optin - (int)at.sharedSizeBytes;
+  *reserved += (int)at.sharedSizeBytes;  // per CTA beside the dynamic part
+  *most = optin - (int)at.sharedSizeBytes;
+  return TRUST_TC_OK;
+}
+
+int batch_count_warp_words(int *words) {
+  int per_sm = 0, reserved = 0, most = 0;
+  int rc = shared_limits(kernel_for(256, true), &per_sm, &reserved, &most);
+  if (rc) return rc;
+  *words = (per_sm / 4 - reserved - 8 * WL_BYTES) / (8 * 4) & ~3;
+  return TRUST_TC_OK;
+}
+
+int batch_count_occupancy(int threads, bool bitmaps, size_t table_bytes, int *blocks_per_sm) {
+  const void *fn = kernel_for(threads, bitmaps);
+  const int smem = (int)smem_for(table_bytes, threads);
+  int per_sm = 0, reserved = 0, most = 0;
+  int rc = shared_limits(fn, &per_sm, &reserved, &most);
+  if (rc) return rc;
   if (smem > most) {
     *blocks_per_sm = 0;
     return TRUST_TC_OK;
   }
+  // (the query honours the carveout an earlier batch has set)
+  TC_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
   TC_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
   TC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fn, threads, smem));
+  // What the resident CTAs leave of the SM's memory is L1 (500 graphs of 20,000 vertices 0.62 -> 0.48 ms, four
+  // of 2 M vertices 1.14 -> 0.65).
+  const int pct = (int)(100.0 * *blocks_per_sm * (smem + reserved) / per_sm) + 1;
+  TC_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, std::min(pct, 100)));
   return TRUST_TC_OK;
 }
 
-int launch_batch_count(const BatchCountArgs &a, int blocks, int threads, cudaStream_t st) {
-  const size_t smem = smem_for((size_t)a.table_bytes, threads);
-  if (threads <= 256) batch_count_kernel<256, 4><<<blocks, threads, smem, st>>>(a);
-  else batch_count_kernel<1024, 1><<<blocks, threads, smem, st>>>(a);
+int launch_batch_count(const BatchCountArgs &a, int blocks, int threads, bool bitmaps, cudaStream_t st) {
+  BatchCountArgs p = a;
+  void *params[] = {&p};
+  TC_CUDA_TRY(cudaLaunchKernel(kernel_for(threads, bitmaps), dim3((unsigned)blocks), dim3((unsigned)threads), params,
+                               smem_for((size_t)a.table_bytes, threads), st));
   TC_NOTE_LAUNCH();
-  TC_CUDA_TRY(cudaGetLastError());
   return TRUST_TC_OK;
 }
 

@@ -19,8 +19,10 @@ struct BatchCountArgs {
   int chunk;                 // steps per queue claim
 };
 
-// Resident CTAs per SM with table_bytes of tables (0: too much shared memory).
-int batch_count_occupancy(int threads, size_t table_bytes, int *blocks_per_sm);
-int launch_batch_count(const BatchCountArgs &a, int blocks, int threads, cudaStream_t st);
+// The most words per warp with which four CTAs of eight warps stay resident on an SM.
+int batch_count_warp_words(int *words);
+// Resident CTAs per SM with table_bytes of tables (0: too much shared memory); the SM's other memory becomes L1.
+int batch_count_occupancy(int threads, bool bitmaps, size_t table_bytes, int *blocks_per_sm);
+int launch_batch_count(const BatchCountArgs &a, int blocks, int threads, bool bitmaps, cudaStream_t st);
 
 }  // namespace tc
