@@ -90,6 +90,50 @@ def test_invalid_input(ctx):
         assert T.count_csr(*_dev(beg, adj), ctx=ctx).triangles == expect
 
 
+@pytest.mark.parametrize("longest", [511, 512, 513, 1025, 16_384, 16_385, 60_000])
+@pytest.mark.parametrize("n,short", [(65_536, 2), (20_000, 40)])
+def test_long_rows(ctx, longest, n, short):
+    """Rows at the bounds of what a warp takes, one or several warps to a row (n, short), that point at each
+    other, with repeated entries, counted or not (slices), unsorted, and with an invalid entry."""
+    rng = np.random.default_rng(longest + n)
+    lens = rng.integers(0, 2 * short, size=n)
+    hubs = rng.choice(n, 5, replace=False)
+    lens[hubs] = (longest, longest - 1, 700, longest, 0)
+    beg = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    adj = rng.integers(0, n, size=int(beg[-1])).astype(np.int32)
+    for h in hubs[:4]:
+        adj[beg[h]:beg[h] + 5] = hubs
+    if adj.size >= 1 << 21:
+        pytest.skip("not a small graph")
+    _same_as_general(ctx, beg, adj, O.count_forward(beg, adj, threads=8))
+    db, da = _dev(beg, adj)
+    cuts = (0, int(hubs[0]), int(hubs[0]) + 1, n)
+    parts = [T.count_csr(db, da, ctx=ctx, row_range=(a, b)) for a, b in zip(cuts[:-1], cuts[1:]) if a < b]
+    assert sum(r.triangles for r in parts) == O.count_forward(beg, adj, threads=8)
+    assert sum(r.wedges for r in parts) == O.wedges(beg, adj)
+    for row_range in (None, (int(hubs[0]) + 1, n)):  # the entry's row is counted, and is only checked
+        bad = da.clone()
+        bad[int(beg[hubs[0]]) + longest // 2] = n
+        with pytest.raises(T.TrustTcError) as e:
+            T.count_csr(db, bad, ctx=ctx, row_range=row_range)
+        assert e.value.status == _lib.E_IDS
+
+
+@pytest.mark.parametrize("splits", [1, 2, 8])
+def test_rows_shared_by_warps_and_long(ctx, splits):
+    """Rows of up to `splits` times a warp's bound stay with their warps, longer ones do not."""
+    n = 2000
+    rng = np.random.default_rng(splits)
+    fill = 16 * n * splits // n + 8 if splits < 8 else 140
+    lens = np.full(n, fill)
+    for k, d in enumerate((512 * splits - 1, 512 * splits, 512 * splits + 1, 512 * splits + 33)):
+        lens[3 * k] = d
+    beg = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    adj = rng.integers(0, n, size=int(beg[-1])).astype(np.int32)
+    assert min(8, max(1, adj.size // (16 * n))) == splits
+    _same_as_general(ctx, beg, adj, O.count_forward(beg, adj, threads=8))
+
+
 def test_first_call_on_a_capturing_stream():
     """A call cannot be captured (it synchronises): it fails, and the context's next call counts."""
     beg, adj = O.build_csr(graphs.complete(60)[0], 60)

@@ -7,6 +7,7 @@
 
 // Device scratch reused across calls (work queues, class lists, spill tables, staging copies of
 // host input).  Replaces the per-call cudaMalloc/cudaFree of Without-graph-partition/TC.cu:647-711.
+constexpr int SMALL_MAX_UNITS = 12288;
 struct trust_tc_ctx {
   int device = -1;
   int num_sms = 0;
@@ -55,6 +56,7 @@ struct trust_tc_ctx {
   size_t split_rowmap_cap = 0;
   int32_t *d_split_adj = nullptr;
   size_t split_adj_cap = 0;
+  int2 *d_small_units = nullptr;  // behind d_small: pieces of long rows
   TcControl *d_small = nullptr;  // behind d_ctl: accumulators of the one-launch path, zero between calls
   unsigned *d_bits_cols = nullptr;  // block-bitmap path: column popularity and ranks, counters, row lists
   size_t bits_cols_cap = 0;
