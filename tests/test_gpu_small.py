@@ -134,6 +134,26 @@ def test_rows_shared_by_warps_and_long(ctx, splits):
     _same_as_general(ctx, beg, adj, O.count_forward(beg, adj, threads=8))
 
 
+@pytest.mark.parametrize("length", [2, 500, 5000, 60_000])
+def test_overlapping_rows_end_early(ctx, length):
+    """Offsets that go back and forth make every other row overlap, with more arcs in all than can be walked:
+    refused at once."""
+    import time
+    n = 60_000
+    beg = np.zeros(n + 1, dtype=np.int64)
+    beg[1::2] = length
+    beg[-1] = 1_900_000
+    beg[-2] = 0
+    adj = np.zeros(1_900_000, dtype=np.int32)
+    db, da = _dev(beg, adj)
+    t = time.perf_counter()
+    with pytest.raises(T.TrustTcError) as e:
+        T.count_csr(db, da, ctx=ctx)
+    assert e.value.status == _lib.E_OFFSETS and time.perf_counter() - t < 5.0
+    ok, tri = graphs.complete(40)
+    assert T.count_csr(*_dev(*O.build_csr(ok, 40)), ctx=ctx).triangles == tri
+
+
 def test_first_call_on_a_capturing_stream():
     """A call cannot be captured (it synchronises): it fails, and the context's next call counts."""
     beg, adj = O.build_csr(graphs.complete(60)[0], 60)

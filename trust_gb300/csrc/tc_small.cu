@@ -220,6 +220,9 @@ __global__ void __launch_bounds__(SM_THREADS, 6) small_kernel(SmallArgs p) {
     int b;
     int d = checked_row(p, v, b);
     if (d < 0) {
+      // Rows that overlap (invalid offsets) can hold far more arcs than the graph, but there is a row out of order
+      // between any two of them: a CTA that meets one claims no more.
+      if (lane == 0) atomicMax(&next, SM_WARPS * tasks);
       bad |= TC_DEV_BAD_OFFSETS;
       continue;
     }
