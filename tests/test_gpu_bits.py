@@ -132,3 +132,50 @@ def test_slice_check_sees_every_row(where, pad):
     lo, hi = n // 2 - 3, n // 2 + 3
     r = T.count_csr(db, da, direction_split=1, row_range=(lo, hi))
     assert r.direction_split == int(where == "none") and r.triangles == _slice_count(beg, adj, lo, hi)
+
+
+def test_slices_of_little_work():
+    """Slices that repay the conversion, that do not by their rows' squares, and that do not by their probes
+    alone (planned for the bitmaps first): a clique and rows that point into it, in a graph of 2 M rows."""
+    n, k = 2_000_000, 800
+    rng = np.random.default_rng(8)
+    rows = {v: np.arange(v + 1, k) for v in range(k)}
+    for v in range(k, 6000):
+        rows[v] = np.unique(np.concatenate([rng.integers(0, k, size=4), rng.integers(k, n, size=3)]))
+    beg, adj = _csr(rows, n)
+    db, da = torch.from_numpy(beg).cuda(), torch.from_numpy(adj).cuda()
+    d = np.diff(beg)
+    with T.Context() as ctx:
+        cuts = [0, 100, 300, k, 3000, n]
+        ranges = [(0, k), (0, 200), (0, 6000), (100, 900)] + list(zip(cuts[:-1], cuts[1:]))
+        for _ in range(2):
+            for lo, hi in ranges:
+                r = T.count_csr(db, da, ctx=ctx, direction_split=1, row_range=(lo, hi))
+                assert r.direction_split == 1
+                assert r.triangles == O.count_forward_sorted_range(beg, adj, lo, hi, 2, 8)
+                at = slice(beg[lo], beg[hi])
+                src = np.repeat(np.arange(lo, hi), d[lo:hi])
+                assert r.wedges == int(np.minimum(d[adj[at]], d[src])[d[src] >= 2].sum())
+
+
+@pytest.mark.parametrize("off", [0, 1, 2, 3])
+@pytest.mark.parametrize("size", [290, 300, 1000, 4099])
+def test_slice_check_on_unaligned_entries(off, size):
+    """The check streams 16 bytes at a time: one descent at every place of small arrays of every alignment."""
+    n = 4100
+    beg = np.zeros(n + 1, dtype=np.int64)
+    beg[n // 2 + 1:] = 280  # row n/2, the slice; the last row holds the rest
+    beg[-1] = size
+    good = np.concatenate([np.arange(280), np.arange(size - 280)]).astype(np.int32)
+    buf = torch.zeros(size + 8, dtype=torch.int32, device="cuda")
+    da, db = buf[off:off + size], torch.from_numpy(beg).cuda()
+    with T.Context() as ctx:
+        places = [None] + [p for p in {281, 282, 283, 284, 285, size - 3, size - 2, size - 1} if 280 < p < size]
+        for at in places:
+            a = good.copy()
+            if at is not None:
+                a[at] = a[at - 1]
+            da.copy_(torch.from_numpy(a))
+            r = T.count_csr(db, da, ctx=ctx, direction_split=1, row_range=(n // 2, n // 2 + 1))
+            assert r.direction_split == int(at is None)
+            assert r.triangles == _slice_count(beg, a, n // 2, n // 2 + 1)

@@ -239,6 +239,14 @@ static bool split_pays(unsigned long long w_all, unsigned long long w_min, int64
   return (double)w_min <= 0.8 * (double)w_all && saved >= 32.0 * (double)(m + n);
 }
 
+// Whether a slice's probes repay the block bitmaps, whose conversion takes the whole graph (9 ps per arc and
+// 0.38 ns per row on GB300) where the two hash passes only take the slice (1.2 ps per probe more, and 0.5 ms
+// for their set-up).  R-MAT 22 (64 M arcs) in quarters to 256ths, ms with bitmaps / hash passes: 3.9 / 13.6 and
+// 3.7 / 3.1 for the first and the last quarter, 1.8 / 1.7 and 2.1 / 1.2 for a 64th; R-MAT 20: bitmaps in every slice.
+static bool slice_repays_bits(unsigned long long probes, int64_t m, int64_t n) {
+  return probes + (1ull << 29) >= 8ull * (unsigned long long)m + 300ull * (unsigned long long)n;
+}
+
 static int split_second_pass(trust_tc_ctx *c, const DevGraph3 &g, const trust_tc_opts &o, bool same,
                              int64_t max_out_degree, trust_tc_result *rb, float *t_build);
 
@@ -305,6 +313,7 @@ static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust
   TcControl *ctl = c->d_ctl;
   // source rows whose arcs are counted (one CSR): [row_lo, row_hi); row_hi = -1 means all rows
   const int64_t row_lo = g.row_lo, row_hi = g.row_hi > 0 ? g.row_hi : -1;
+  const bool slice = row_lo > 0 || (row_hi >= 0 && row_hi < g.rows);
   TC_CUDA_TRY(cudaEventRecord(c->ev[0], st));
   // a small graph under the default schedule and launch shape: everything in one launch (the direction
   // split, cycle recording and the hub kernel's own options keep the general path)
@@ -340,6 +349,7 @@ static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust
   const bool small_alt = fused && o.schedule == TRUST_TC_SCHED_LEARNED && o.warp_max_degree <= 0 &&
                          o.direction_split != 1 && g.min_deg == 2 && g.mA < TC_SMALL_SKEWED_ARCS &&
                          14 * g.rows < ((int64_t)1 << 31);
+  const bool slice_squares = slice && o.direction_split == 1 && !slice_repays_bits(0, g.mA, g.rows);
   if (fused) {
     rc = ensure((void **)&c->d_lists, &c->lists_cap,
                 sizeof(int) * (size_t)std::max<int64_t>((small_alt ? 14 : 7) * g.rows, 1));
@@ -349,6 +359,7 @@ static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust
                                o.schedule, ctl, c->d_lists, c->num_sms, st, row_lo, row_hi,
                                small_alt ? c->d_lists + 7 * g.rows : nullptr);
     if (rc) return rc;
+    if (slice_squares && (rc = launch_slice_work(g.begA, row_lo, row_hi, ctl, c->num_sms, st))) return rc;
   } else {
     // 1. validation of every distinct CSR: offsets always, ids on request
     const int64_t rowsA = g.rowmap ? g.rowsA : g.rows;
@@ -403,7 +414,7 @@ static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust
   // with the split (of one graph or of a tile job, below), rows longer than BITS_TABLE_MIN are counted as
   // block bitmaps (tc_bits.cu) unless
   // the caller asks for something of the hash tables' own: cycles, hub clusters, CTA bounds below
-  const bool bits_ok = !o.record_cycles && o.hub_cluster == 0 && !o.test_wait_expiry &&
+  bool bits_ok = !o.record_cycles && o.hub_cluster == 0 && !o.test_wait_expiry &&
                        cfg.cta_max >= BITS_TABLE_MIN && bits_eligible(g, h.max_out_degree);
   unsigned long long plan_wedges = 0;
   BitsPlan bits;
@@ -424,6 +435,8 @@ static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust
   };
   if (consider) {
     *planned = true;
+    // (the squares are known before the pass, the probes, never more, after it)
+    if (slice_squares && fused && !slice_repays_bits(h.slice_work, g.mA, g.rows)) bits_ok = false;
     const float *d_model = nullptr;
     if (learned) {
       rc = load_model(c, o.model, &d_model);
@@ -466,12 +479,21 @@ static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust
       split = sorted && split_pays(plan.w_all, plan.w_min, g.mA, g.rows);
     }
     // the pass has checked the slice's rows; its arcs lead to rows outside it, which have to be
-    // duplicate-free as well (the whole graph's check: 0.3 ms for 170 M arcs)
-    if (split && (row_lo > 0 || (row_hi >= 0 && row_hi < g.rows))) {
+    // duplicate-free as well (the whole graph's check: 0.15 ms for 185 M arcs)
+    if (split && slice) {
       bool increasing = false;
       rc = rows_increasing(c, g.begA, g.adjA, g.rows, g.mA, st, &increasing);
       if (rc) return rc;
       split = increasing;
+    }
+    if (split && bits_ok && slice && !slice_repays_bits(plan.w_min, g.mA, g.rows)) {
+      bits_ok = false;  // the hash passes' plan instead (classes and decisions stay)
+      rc = split_plan(c, g.begA, g.adjA, g.rows, g.mA, st, nullptr, cfg.warp_max, cfg.cta_max, TC_PROMOTE_LOG2,
+                      cfg.threads / 32, ctl, row_lo, row_hi, 0);
+      if (rc) return rc;
+      TC_CUDA_TRY(cudaStreamSynchronize(st));
+      split_plan_read(c, &plan);
+      if (plan.overflow) return TRUST_TC_E_DEVICE;
     }
     if (split && bits_ok) {
       plan_wedges = plan.w_min;

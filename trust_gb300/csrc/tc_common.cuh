@@ -47,6 +47,7 @@ struct TcControl {
   int class_off[TC_NUM_CLASSES];      // list offsets, when computed on the device (batches)
   unsigned long long long_arcs;       // arcs of rows longer than TC_LONG_ROW (single-graph calls)
   int class_count_alt[TC_NUM_CLASSES];  // small graphs: list sizes under the plain split as well
+  unsigned long long slice_work;      // slices with the split: no fewer than its probes (squared row lengths)
 };
 constexpr int TC_LONG_ROW = 128;
 

@@ -170,6 +170,8 @@ int split_build(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t
 // The split plan of a job over three CSRs (tile jobs): probe totals and the arcs of B to move,
 // read back like split_plan's.
 int tile_split_plan(trust_tc_ctx *c, const DevGraph3 &g, cudaStream_t st, int table_min);
+// ctl->slice_work += the squares of the lengths of rows [row_lo, row_hi): no fewer than a split's probes there.
+int launch_slice_work(const int64_t *beg, int64_t row_lo, int64_t row_hi, TcControl *ctl, int num_sms, cudaStream_t st);
 // Whether every row of a CSR is strictly increasing (so duplicate-free); synchronous.
 int rows_increasing(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t rows, int64_t m, cudaStream_t st,
                     bool *out);

@@ -678,17 +678,23 @@ __global__ void __launch_bounds__(256) rows_increasing_kernel(const int64_t *__r
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   long long n = 0;
-  for (int64_t i = tid; i + 1 < m; i += 4 * stride) {
-    int x[4], y[4];
+  // 16-byte loads from the first boundary on, each with the entry that follows; single pairs before and after
+  const int64_t lead = min((int64_t)(((16u - ((unsigned)(uintptr_t)adj & 15u)) & 15u) >> 2), m);
+  const int64_t n4 = (m - lead) >> 2, rest = lead + 4 * n4;
+  for (int64_t i = tid; i < n4; i += 2 * stride) {
+    int4 x[2];
+    int y[2];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int64_t k = i + r * stride;
-      x[r] = k + 1 < m ? tc_ld_nc(adj + k) : 0;
-      y[r] = k + 1 < m ? tc_ld_nc(adj + k + 1) : 1;
+    for (int r = 0; r < 2; ++r) {
+      const int64_t k = i + r * stride, at = lead + 4 * k;
+      x[r] = k < n4 ? __ldg(reinterpret_cast<const int4 *>(adj + at)) : make_int4(0, 1, 2, 3);
+      y[r] = k < n4 && at + 4 < m ? tc_ld_nc(adj + at + 4) : 0x7fffffff;
     }
 #pragma unroll
-    for (int r = 0; r < 4; ++r) n += x[r] >= y[r];
+    for (int r = 0; r < 2; ++r) n += (x[r].x >= x[r].y) + (x[r].y >= x[r].z) + (x[r].z >= x[r].w) + (x[r].w >= y[r]);
   }
+  if (tid < lead && tid + 1 < m) n += tc_ld_nc(adj + tid) >= tc_ld_nc(adj + tid + 1);
+  for (int64_t k = rest + tid; k + 1 < m; k += stride) n += tc_ld_nc(adj + k) >= tc_ld_nc(adj + k + 1);
   for (int64_t v = tid; v < rows; v += stride) {
     const long long b = tc_ld_nc(beg + v), e = tc_ld_nc(beg + v + 1);
     if (b < e && e > 0 && e < m) n -= tc_ld_nc(adj + e - 1) >= tc_ld_nc(adj + e);
@@ -698,6 +704,26 @@ __global__ void __launch_bounds__(256) rows_increasing_kernel(const int64_t *__r
   if ((threadIdx.x & 31) == 0 && n) atomicAdd(excess, (unsigned long long)n);
 }
 
+__global__ void __launch_bounds__(256) slice_work_kernel(const int64_t *__restrict__ beg, int64_t row_lo, int64_t row_hi,
+                                                         unsigned long long *work) {
+  unsigned long long n = 0;
+  for (int64_t v = row_lo + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < row_hi; v += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned long long d = (unsigned long long)(tc_ld_nc(beg + v + 1) - tc_ld_nc(beg + v));
+    n += d * d;
+  }
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) n += __shfl_down_sync(TC_FULL_MASK, n, o);
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(work, n);
+}
+
+int launch_slice_work(const int64_t *beg, int64_t row_lo, int64_t row_hi, TcControl *ctl, int num_sms, cudaStream_t st) {
+  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((row_hi - row_lo + 1023) / 1024, (int64_t)num_sms * 4));
+  slice_work_kernel<<<blocks, 256, 0, st>>>(beg, row_lo, row_hi, &ctl->slice_work);
+  TC_NOTE_LAUNCH();
+  TC_CUDA_TRY(cudaGetLastError());
+  return TRUST_TC_OK;
+}
+
 int rows_increasing(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t rows, int64_t m, cudaStream_t st,
                     bool *out) {
   int rc = ensure((void **)&c->d_split_plans, &c->split_plans_cap, TC_PLAN_WORDS * sizeof(unsigned long long));
@@ -705,7 +731,7 @@ int rows_increasing(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int
   unsigned long long *excess = c->d_split_plans + PLAN_UNSORTED;  // beside a plan's totals
   TC_CUDA_TRY(cudaMemsetAsync(excess, 0, sizeof(unsigned long long), st));
   const int blocks =
-      (int)std::max<int64_t>(1, std::min<int64_t>((std::max(rows, m / 4) + 255) / 256, (int64_t)c->num_sms * 16));
+      (int)std::max<int64_t>(1, std::min<int64_t>((std::max(rows, m / 8) + 255) / 256, (int64_t)c->num_sms * 16));
   rows_increasing_kernel<<<blocks, 256, 0, st>>>(beg, adj, rows, m, excess);
   TC_NOTE_LAUNCH();
   TC_CUDA_TRY(cudaGetLastError());
