@@ -179,3 +179,21 @@ def test_slice_check_on_unaligned_entries(off, size):
             r = T.count_csr(db, da, ctx=ctx, direction_split=1, row_range=(n // 2, n // 2 + 1))
             assert r.direction_split == int(at is None)
             assert r.triangles == _slice_count(beg, a, n // 2, n // 2 + 1)
+
+
+@pytest.mark.parametrize("n", [425_984, 425_985, 2_000_000])
+@pytest.mark.parametrize("popular", [0, 1000])
+def test_wide_graphs(n, popular):
+    """More columns than two bitmaps hold: entries spread over all of them (hash passes), or most of them in
+    a few popular ones; one graph and tile jobs."""
+    rng = np.random.default_rng(n + popular)
+    hubs, row = 30, 700
+    rows = {h: np.unique(np.concatenate([np.arange(h + 1, hubs), rng.integers(hubs, n, size=row)])) for h in range(hubs)}
+    for v in range(hubs, n, 40):
+        own = rng.integers(hubs, n, size=rng.integers(1, 6))
+        rows[v] = np.unique(np.concatenate([own, rng.integers(0, popular, size=20)]) if popular else own)
+    beg, adj = _csr(rows, n)
+    _check(beg, adj)
+    db, da = torch.from_numpy(beg).cuda(), torch.from_numpy(adj).cuda()
+    r = T.count_tiles(db, da, 2, direction_split=1)
+    assert r.triangles == O.count_forward_sorted_range(beg, adj, 0, n, 2, 8) and r.direction_split >= 1

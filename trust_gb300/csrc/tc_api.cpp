@@ -437,6 +437,8 @@ static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust
     *planned = true;
     // (the squares are known before the pass, the probes, never more, after it)
     if (slice_squares && fused && !slice_repays_bits(h.slice_work, g.mA, g.rows)) bits_ok = false;
+    // (without being told to, no graph measured whose columns do not suit the bitmaps is split: little is saved there)
+    if (bits_ok && o.direction_split == 1 && (rc = bits_columns(c, g, st, &bits, &bits_ok))) return rc;
     const float *d_model = nullptr;
     if (learned) {
       rc = load_model(c, o.model, &d_model);
@@ -510,6 +512,7 @@ static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust
                            h.max_out_degree >= 64 && g.mB >= TC_LEARNED_MIN_ARCS));
   if (consider3) {
     *planned = true;
+    if (bits_ok && o.direction_split == 1 && (rc = bits_columns(c, g, st, &bits, &bits_ok))) return rc;
     rc = tile_split_plan(c, g, st, bits_ok ? BITS_TABLE_MIN : 0);
     if (rc) return rc;
     TC_CUDA_TRY(cudaStreamSynchronize(st));

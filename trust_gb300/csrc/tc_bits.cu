@@ -76,25 +76,36 @@ __global__ void __launch_bounds__(256) rank_hist_kernel(const u32 *__restrict__ 
   counts[(size_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// rank[w] = position of column w, popular buckets first (any order inside a bucket and tile).
+// rank[w] = position of column w, popular buckets first (any order inside a bucket and tile).  seen (or
+// null): sampled entries whose column has a rank below `direct`, and all of them.
 __global__ void __launch_bounds__(256) rank_scatter_kernel(const u32 *__restrict__ indeg, int64_t n,
                                                            const u32 *__restrict__ offs, u32 ntiles,
-                                                           u32 *__restrict__ rank) {
+                                                           u32 *__restrict__ rank, u32 direct, u32 *seen) {
   __shared__ u32 cur[256];
   cur[threadIdx.x] = offs[(size_t)threadIdx.x * ntiles + blockIdx.x];
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int64_t base = (int64_t)blockIdx.x * RK_TILE;
+  u32 in = 0, all = 0;
   for (int r = 0; r < RK_TILE / 256; ++r) {
     const int64_t i = base + r * 256 + threadIdx.x;
-    const int b = i < n ? pop_bucket(indeg[i]) : 256;
+    const u32 entries = i < n ? indeg[i] : 0u;
+    const int b = i < n ? pop_bucket(entries) : 256;
     const unsigned peers = __match_any_sync(TC_FULL_MASK, b);
     const int leader = __ffs(peers) - 1;
     u32 at = 0;
     if (b < 256 && lane == leader) at = atomicAdd(&cur[b], (u32)__popc(peers));
     at = __shfl_sync(TC_FULL_MASK, at, leader);
-    if (b < 256) rank[i] = at + __popc(peers & tc_lanemask_lt());
+    at += __popc(peers & tc_lanemask_lt());
+    if (b < 256) rank[i] = at;
+    if (at < direct) in += entries;
+    all += entries;
   }
+  if (!seen) return;
+  in = __reduce_add_sync(TC_FULL_MASK, in);
+  all = __reduce_add_sync(TC_FULL_MASK, all);
+  if (lane == 0 && in) atomicAdd(seen, in);
+  if (lane == 0 && all) atomicAdd(seen + 1, all);
 }
 
 // ---- rows to blocks --------------------------------------------------------------------------
@@ -636,14 +647,86 @@ bool bits_eligible(const DevGraph3 &g, int64_t max_out_degree) {
   return max_out_degree > BITS_TABLE_MIN && max_out_degree <= BITS_MAX_ROW && words < ((int64_t)1 << 32);
 }
 
+// The scratch block of both steps: in-degrees, ranks, rank histogram and its scan, counters (units, in-list
+// entries, claims, warp rows and CTA rows of either CSR, then sampled entries), row lists.
+namespace {
+struct Columns {
+  u32 *indeg, *rank, *counts, *scratch, *ctr;
+  int *longs;
+  int64_t cols;
+  u32 ntiles;
+  int nb;
+};
+constexpr int CTR_SEEN = 8;
+}  // namespace
+
+static bool is_tile(const DevGraph3 &g) { return g.begA != g.begB || g.adjA != g.adjB || !one_csr(g); }
+
+static int columns_of(trust_tc_ctx *c, const DevGraph3 &g, Columns *k) {
+  k->cols = is_tile(g) ? g.boundA : g.rows;
+  k->nb = (int)std::min<int64_t>((((k->cols + 15) / 16) + 7) & ~7ll, BITS_MAX_BLOCKS);
+  k->ntiles = (u32)((k->cols + RK_TILE - 1) / RK_TILE);
+  const size_t nn = (size_t)k->cols, hist = 256 * (size_t)k->ntiles, scan = scan_u32_scratch(256 * (int64_t)k->ntiles);
+  const size_t rows = (size_t)std::max(g.rows, one_csr(g) ? 0 : g.rowsC);
+  int rc = ensure((void **)&c->d_bits_cols, &c->bits_cols_cap, sizeof(u32) * (2 * nn + rows + hist + scan + 16));
+  if (rc) return rc;
+  k->indeg = c->d_bits_cols;
+  k->rank = k->indeg + nn;
+  k->counts = k->rank + nn;
+  k->scratch = k->counts + hist;
+  k->ctr = k->scratch + scan;
+  k->longs = reinterpret_cast<int *>(k->ctr + 16);
+  return TRUST_TC_OK;
+}
+
+// Rank the columns by popularity.
+static int rank_columns(trust_tc_ctx *c, const DevGraph3 &g, const Columns &k, bool count_seen, cudaStream_t st) {
+  int rc;
+  TC_CUDA_TRY(cudaMemsetAsync(k.indeg, 0, sizeof(u32) * (size_t)k.cols, st));
+  TC_CUDA_TRY(cudaMemsetAsync(k.ctr, 0, sizeof(u32) * 16, st));
+  indeg_kernel<<<blocks_for(g.mA, 1024, c->num_sms, 16), 256, 0, st>>>(g.adjA, g.mA, k.indeg);
+  note_launch();
+  if (!one_csr(g)) {
+    indeg_kernel<<<blocks_for(g.mC, 1024, c->num_sms, 16), 256, 0, st>>>(g.adjC, g.mC, k.indeg);
+    note_launch();
+  }
+  rank_hist_kernel<<<k.ntiles, 256, 0, st>>>(k.indeg, k.cols, k.counts, k.ntiles);
+  TC_CUDA_TRY(cudaGetLastError());
+  note_launch();
+  if ((rc = scan_exclusive_u32(k.counts, k.counts, 256 * (int64_t)k.ntiles, k.scratch, st))) return rc;
+  rank_scatter_kernel<<<k.ntiles, 256, 0, st>>>(k.indeg, k.cols, k.counts, k.ntiles, k.rank, 16u * (u32)k.nb,
+                                                count_seen ? k.ctr + CTR_SEEN : nullptr);
+  TC_CUDA_TRY(cudaGetLastError());
+  note_launch();
+  return TRUST_TC_OK;
+}
+
+// A bitmap over 212,992 of many columns of about equal popularity leaves most entries to the tails'
+// hash sets, one load and lookup each.  Share of the sampled entries in the bitmap, and ms with block bitmaps /
+// hash passes, Erdos-Renyi of 600,000 vertices 0.62, 46 / 56; 800,000 0.51, 43 / 42; 1 M 0.41, 64 / 57; 4 M 0.14,
+// 110 / 77.  Skewed graphs: R-MAT 24 with a = 0.45 0.67, 53 / 67, with a = 0.70 0.98, 44 / 170.
+constexpr double BITS_MIN_SEEN = 0.5;
+
+int bits_columns(trust_tc_ctx *c, const DevGraph3 &g, cudaStream_t st, BitsPlan *plan, bool *suit) {
+  Columns k;
+  int rc = columns_of(c, g, &k);
+  if (rc) return rc;
+  *suit = true;
+  if ((double)k.cols * BITS_MIN_SEEN <= 16.0 * k.nb) return TRUST_TC_OK;  // whatever their popularity
+  if ((rc = rank_columns(c, g, k, true, st))) return rc;
+  u32 seen[2];
+  TC_CUDA_TRY(cudaMemcpyAsync(seen, k.ctr + CTR_SEEN, sizeof seen, cudaMemcpyDeviceToHost, st));
+  TC_CUDA_TRY(cudaStreamSynchronize(st));
+  *suit = (double)seen[0] >= BITS_MIN_SEEN * (double)seen[1];
+  plan->ranked = true;
+  return TRUST_TC_OK;
+}
+
 // Enqueue the conversion and the work units (after the scheduling pass and its readback).
 int bits_prepare(trust_tc_ctx *c, const DevGraph3 &g, int64_t row_lo, int64_t row_hi, const SchedPlan &plan,
                  int64_t max_out_degree, cudaStream_t st, BitsPlan *out) {
-  const bool tile = g.begA != g.begB || g.adjA != g.adjB || !one_csr(g);
+  const bool tile = is_tile(g);
   const bool two = !one_csr(g);  // rows of two CSRs are converted
-  const int64_t cols = tile ? g.boundA : g.rows;
-  const int nb = (int)std::min<int64_t>((((cols + 15) / 16) + 7) & ~7ll, BITS_MAX_BLOCKS);
-  const u32 ntiles = (u32)((cols + RK_TILE - 1) / RK_TILE);
   // units: every table at least one, and one more per `target` probes: about eight units per resident
   // CTA, so the last ones end together, but not so small that a unit's set-up shows (R-MAT 18: 1.63 ms
   // at 2^18 probes, 1.81 at 2^20; R-MAT 25: 426 and 415)
@@ -654,41 +737,21 @@ int bits_prepare(trust_tc_ctx *c, const DevGraph3 &g, int64_t row_lo, int64_t ro
   const int64_t rows_c = two ? g.rowsC : 0;
   const u32 base_c = (u32)((g.mA + 6 * g.rows + 11) & ~3ll);
   const size_t words = two ? (size_t)base_c + (size_t)(g.mC + 6 * g.rowsC + 8) : (size_t)(g.mA + 6 * g.rows + 8);
-  // one scratch block: in-degrees, ranks, rank histogram, counters, row lists
-  const size_t nn = (size_t)cols;
-  const size_t hist = 256 * (size_t)ntiles;
-  int rc;
-  if ((rc = ensure((void **)&c->d_bits_cols, &c->bits_cols_cap,
-                   sizeof(u32) * (2 * nn + (size_t)std::max(g.rows, rows_c) + hist +
-                                  scan_u32_scratch(256 * (int64_t)ntiles) + 16))))
-    return rc;
+  Columns k;
+  int rc = columns_of(c, g, &k);
+  if (rc) return rc;
   if ((rc = ensure((void **)&c->d_bits_desc, &c->bits_desc_cap, sizeof(int4) * (size_t)(g.rows + rows_c)))) return rc;
   if ((rc = ensure((void **)&c->d_bits_ent, &c->bits_ent_cap, sizeof(u32) * words))) return rc;
   if ((rc = ensure((void **)&c->d_bits_units, &c->bits_units_cap, sizeof(Unit) * (size_t)max_units))) return rc;
   if ((rc = ensure((void **)&c->d_split_adj, &c->split_adj_cap, sizeof(int32_t) * (size_t)std::max<int64_t>(g.mB, 1))))
     return rc;
-  u32 *indeg = c->d_bits_cols, *rank = indeg + nn, *counts = rank + nn;
-  u32 *scratch = counts + hist;
-  // units, in-list entries, claims, then warp rows and CTA rows of either CSR
-  u32 *ctr = scratch + scan_u32_scratch(256 * (int64_t)ntiles);
-  int *longs = reinterpret_cast<int *>(ctr + 16);
+  if (!out->ranked && (rc = rank_columns(c, g, k, false, st))) return rc;
+  u32 *const rank = k.rank, *const ctr = k.ctr;
+  int *const longs = k.longs;
+  const int nb = k.nb;
   int4 *desc = reinterpret_cast<int4 *>(c->d_bits_desc);
   int4 *desc_c = two ? desc + g.rows : desc;
   Unit *units = reinterpret_cast<Unit *>(c->d_bits_units);
-  TC_CUDA_TRY(cudaMemsetAsync(indeg, 0, sizeof(u32) * nn, st));
-  TC_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(u32) * 16, st));
-  indeg_kernel<<<blocks_for(g.mA, 1024, c->num_sms, 16), 256, 0, st>>>(g.adjA, g.mA, indeg);
-  note_launch();
-  if (two) {
-    indeg_kernel<<<blocks_for(g.mC, 1024, c->num_sms, 16), 256, 0, st>>>(g.adjC, g.mC, indeg);
-    note_launch();
-  }
-  rank_hist_kernel<<<ntiles, 256, 0, st>>>(indeg, cols, counts, ntiles);
-  TC_CUDA_TRY(cudaGetLastError());
-  note_launch();
-  if ((rc = scan_exclusive_u32(counts, counts, 256 * (int64_t)ntiles, scratch, st))) return rc;
-  rank_scatter_kernel<<<ntiles, 256, 0, st>>>(indeg, cols, counts, ntiles, rank);
-  note_launch();
   auto convert = [&](const int64_t *beg, const int32_t *adj, int64_t n, u32 base, int4 *d, u32 *nlongs) -> int {
     bits_short_kernel<<<blocks_for(n, 256, c->num_sms, 32), 256, 0, st>>>(beg, adj, n, rank, nb, base, c->d_bits_ent, d,
                                                                           longs, nlongs);

@@ -15,9 +15,12 @@ struct BitsPlan {
   int nb = 0;               // blocks (of 16 columns) of the bitmap
   unsigned *ctr = nullptr;  // device counters: units, in-list entries, unit claims
   int64_t rows_c_at = 0;    // first C row among the row descriptors
+  bool ranked = false;      // the columns are ranked already (bits_columns)
 };
 
 bool bits_eligible(const DevGraph3 &g, int64_t max_out_degree);
+// Whether enough of the entries fall into the bitmap's columns (waits for st).
+int bits_columns(trust_tc_ctx *c, const DevGraph3 &g, cudaStream_t st, BitsPlan *plan, bool *suit);
 // After the scheduling pass (its pairs, counts and, for one graph, work sums) and its readback.  Only arcs
 // of source rows in [row_lo, row_hi) are counted.  A tile job's A and C rows must be duplicate-free.
 int bits_prepare(trust_tc_ctx *c, const DevGraph3 &g, int64_t row_lo, int64_t row_hi, const SchedPlan &plan,
