@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "tc_batch_count.h"
+#include "tc_rows.cuh"
 
 namespace tc {
 
@@ -23,18 +24,6 @@ struct IdSpace {
 };
 
 // ---- row sets: set.of(lane of the arc).has(entry); no entry (-1) is in no set --------------------
-// Open addressing over 2^log2 slots (log2 >= 6) in buckets of four; -1 = empty.
-__device__ __forceinline__ bool set_insert(int *tab, int log2, int key) {
-  const unsigned mask = (1u << log2) - 1u;
-  unsigned h = tc_hash((unsigned)key, log2 - 2) << 2;
-  for (unsigned it = 0; it <= mask; ++it) {
-    const int prev = atomicCAS(tab + h, -1, key);
-    if (prev == -1 || prev == key) return true;
-    h = (h + 1u) & mask;
-  }
-  return false;
-}
-
 struct HashSet {
   const int *tab;
   int log2;
@@ -163,40 +152,6 @@ __device__ __forceinline__ void probe_chunks(const int32_t *__restrict__ adj, in
 
 // ---- rows of at most 8 entries: each lane walks its own arc's target row against its vertex's keys
 // held in registers -------------------------------------------------------------------------------
-template <int G>
-__device__ __forceinline__ unsigned match_keys(int w, const int (&key)[G]) {
-  bool m = false;
-#pragma unroll
-  for (int k = 0; k < G; ++k) m |= w == key[k];
-  return m;
-}
-
-// The first eight entries and the next four are loaded before any is matched (most rows are that
-// short), then four at a time with the next four in flight.  -2 marks entries past the row.
-template <int G>
-__device__ __forceinline__ unsigned lane_walk(const int32_t *__restrict__ row, int d, const int (&key)[G]) {
-  unsigned h = 0;
-  int w[8];
-#pragma unroll
-  for (int r = 0; r < 8; ++r) w[r] = r < d ? tc_ld_nc(row + r) : -2;
-  int n0 = -2, n1 = -2, n2 = -2, n3 = -2;
-  if (d > 8) {
-    n0 = tc_ld_nc(row + 8);
-    n1 = 9 < d ? tc_ld_nc(row + 9) : -2;
-    n2 = 10 < d ? tc_ld_nc(row + 10) : -2;
-    n3 = 11 < d ? tc_ld_nc(row + 11) : -2;
-  }
-#pragma unroll
-  for (int r = 0; r < 8; ++r) h += match_keys<G>(w[r], key);
-  for (int k = 8; k < d; k += 4) {
-    const int m0 = k + 4 < d ? tc_ld_nc(row + k + 4) : -2, m1 = k + 5 < d ? tc_ld_nc(row + k + 5) : -2,
-              m2 = k + 6 < d ? tc_ld_nc(row + k + 6) : -2, m3 = k + 7 < d ? tc_ld_nc(row + k + 7) : -2;
-    h += match_keys<G>(n0, key) + match_keys<G>(n1, key) + match_keys<G>(n2, key) + match_keys<G>(n3, key);
-    n0 = m0; n1 = m1; n2 = m2; n3 = m3;
-  }
-  return h;
-}
-
 constexpr int LANE_ROW = 128;  // longer target rows are walked by the whole warp
 
 template <int G>
@@ -226,16 +181,6 @@ struct BlockShared {
   int item;
   int next_batch;
 };
-
-__device__ __forceinline__ int ceil_log2_table(int d) {  // smallest power of two >= 2d, at least 64 slots
-  return 32 - __clz(max(2 * d, 64) - 1);
-}
-
-__device__ __forceinline__ void row_of(const int64_t *__restrict__ beg, int v, int &b, int &d) {
-  const long long lo = tc_ld_nc(beg + v), hi = tc_ld_nc(beg + v + 1);
-  b = (int)lo;
-  d = (int)(hi - lo);
-}
 
 __device__ __forceinline__ const int *class_list(const BatchCountArgs &p, int c) { return p.lists + p.ctl->class_off[c]; }
 

@@ -21,6 +21,7 @@
 #include "tc_bits.h"
 #include "tc_count.h"
 #include "tc_internal.h"
+#include "tc_rows.cuh"
 
 namespace tc {
 
@@ -113,21 +114,6 @@ __global__ void __launch_bounds__(256) rank_scatter_kernel(const u32 *__restrict
 // entries that pad its blocks to a multiple of four (m + 6 n entries in all).
 __host__ __device__ __forceinline__ u32 row_start(int64_t beg, int64_t v) { return (u32)((beg + 6 * v + 3) & ~3ll); }
 
-// Position (0..31) of the n-th (0-based) set bit of mask; mask must have more than n set bits.
-__device__ __forceinline__ int nth_bit(unsigned mask, int n) {
-  int pos = 0;
-#pragma unroll
-  for (int step = 16; step >= 1; step >>= 1) {
-    const int cnt = __popc(mask & ((1u << step) - 1u));
-    if (n >= cnt) {
-      n -= cnt;
-      mask >>= step;
-      pos += step;
-    }
-  }
-  return pos;
-}
-
 // Place of a row's e-th block (of nd4 * 4, padding included).  Blocks are laid out in chunks of 32,
 // transposed: eight lanes read a chunk with one 16-byte load each, and the c-th 16-bit lookups of
 // the eight then go to consecutive blocks, whose words share few banks where a row is dense.
@@ -187,7 +173,7 @@ __global__ void __launch_bounds__(256) bits_short_kernel(const int64_t *__restri
       const unsigned starts = __reduce_or_sync(TC_FULL_MASK, in ? 1u << (excl - base) : 0u);
       const int wend = __reduce_max_sync(TC_FULL_MASK, in ? incl : 0);
       const bool valid = lane < wend - base;
-      const int own = valid ? nth_bit(inm, __popc(starts & upto) - 1) : 0;
+      const int own = valid ? nth_set_bit(inm, __popc(starts & upto) - 1) : 0;
       const int bj = __shfl_sync(TC_FULL_MASK, b, own);
       const int ex = __shfl_sync(TC_FULL_MASK, excl, own) - base;
       const int dj = __shfl_sync(TC_FULL_MASK, sd, own);
@@ -369,7 +355,6 @@ __global__ void __launch_bounds__(256) bits_units_kernel(const int64_t *__restri
                                                          const unsigned long long *__restrict__ wsum, u32 *ctr,
                                                          unsigned long long target, Unit *__restrict__ units, int side) {
   const int lane = threadIdx.x & 31;
-  const unsigned lt = tc_lanemask_lt();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t v0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); v0 < n; v0 += stride) {
     const int64_t v = v0 + lane;
@@ -416,7 +401,6 @@ __global__ void __launch_bounds__(256) bits_units_kernel(const int64_t *__restri
     const u32 per = k ? (len + k - 1) / k : 0;
     for (int j = 0; j < k; ++j)
       units[ak + j] = Unit{(int)v, (int)min((u32)j * per, len), (int)min((u32)(j + 1) * per, len), na, (u32)b, ab, side, 0};
-    (void)lt;
   }
 }
 

@@ -23,6 +23,7 @@
 #include <cooperative_groups.h>
 
 #include "tc_count.h"
+#include "tc_rows.cuh"
 
 namespace tc {
 
@@ -33,17 +34,6 @@ namespace tc {
 // is the first slot of bucket hash(key); insertion takes the first free slot from there on
 // (linear probing over slots), so a lookup that finds an empty slot in a bucket without the key
 // can stop: the key would have been placed there.
-__device__ __forceinline__ bool set_insert(int *tab, int log2, int key) {
-  const unsigned mask = (1u << log2) - 1u;
-  unsigned h = tc_hash((unsigned)key, log2 - 2) << 2;
-  for (unsigned it = 0; it <= mask; ++it) {
-    int prev = atomicCAS(tab + h, -1, key);
-    if (prev == -1 || prev == key) return true;
-    h = (h + 1u) & mask;
-  }
-  return false;
-}
-
 __device__ __forceinline__ int set_probe(const int *tab, int log2, int key) {
   const unsigned bmask = (1u << (log2 - 2)) - 1u;
   unsigned b = tc_hash((unsigned)key, log2 - 2);
@@ -223,21 +213,6 @@ struct LongRow {
   static constexpr int value = G;
 };
 
-// Position (0..31) of the n-th (0-based) set bit of mask; mask must have more than n set bits.
-__device__ __forceinline__ int nth_set_bit(unsigned mask, int n) {
-  int pos = 0;
-#pragma unroll
-  for (int step = 16; step >= 1; step >>= 1) {
-    const int cnt = __popc(mask & ((1u << step) - 1u));
-    if (n >= cnt) {
-      n -= cnt;
-      mask >>= step;
-      pos += step;
-    }
-  }
-  return pos;
-}
-
 // Membership of w in the source row of group g of this warp.  G <= 8: the rows are staged in
 // shared memory as G keys per group (-1 past the row), read with 16-byte loads.  G >= 16: each
 // group owns a 4G-slot hash table.
@@ -255,42 +230,6 @@ __device__ __forceinline__ int group_has(const int *wtab, int g, int w) {
     constexpr int LOG2 = (G == 16 ? 4 : 5) + 2;
     return set_probe(wtab + g * (4 * G), LOG2, w);
   }
-}
-
-// Membership of w in a row of at most G keys held in registers (-1 past the row; w >= 0).
-template <int G>
-__device__ __forceinline__ unsigned match_keys(int w, const int (&key)[G]) {
-  bool m = false;
-#pragma unroll
-  for (int k = 0; k < G; ++k) m |= w == key[k];
-  return m;
-}
-
-// One lane walks its own arc's target row against its vertex's keys in registers: the first eight
-// entries and the next four are loaded before any is matched (most of these rows are that short),
-// then four at a time with the next four in flight.  -2 marks entries past the row.
-template <int G>
-__device__ __forceinline__ unsigned lane_walk(const int32_t *__restrict__ row, int d, const int (&key)[G]) {
-  unsigned h = 0;
-  int w[8];
-#pragma unroll
-  for (int r = 0; r < 8; ++r) w[r] = r < d ? tc_ld_nc(row + r) : -2;
-  int n0 = -2, n1 = -2, n2 = -2, n3 = -2;
-  if (d > 8) {
-    n0 = tc_ld_nc(row + 8);
-    n1 = 9 < d ? tc_ld_nc(row + 9) : -2;
-    n2 = 10 < d ? tc_ld_nc(row + 10) : -2;
-    n3 = 11 < d ? tc_ld_nc(row + 11) : -2;
-  }
-#pragma unroll
-  for (int r = 0; r < 8; ++r) h += match_keys<G>(w[r], key);
-  for (int k = 8; k < d; k += 4) {
-    const int m0 = k + 4 < d ? tc_ld_nc(row + k + 4) : -2, m1 = k + 5 < d ? tc_ld_nc(row + k + 5) : -2,
-              m2 = k + 6 < d ? tc_ld_nc(row + k + 6) : -2, m3 = k + 7 < d ? tc_ld_nc(row + k + 7) : -2;
-    h += match_keys<G>(n0, key) + match_keys<G>(n1, key) + match_keys<G>(n2, key) + match_keys<G>(n3, key);
-    n0 = m0; n1 = m1; n2 = m2; n3 = m3;
-  }
-  return h;
 }
 
 // Probe every wedge of a warp whose lanes hold one arc each, lanes [gG, gG+G) belonging to
@@ -760,21 +699,8 @@ __device__ __forceinline__ void walk_row_warp(const int32_t *__restrict__ row, i
   hits += h;
 }
 
-__device__ __forceinline__ int ceil_log2_table(int d) {
-  // smallest power of two >= 2d, at least 64 slots
-  int need = max(2 * d, 64);
-  return 32 - __clz(need - 1);
-}
-
 // Table row (in A) of work row v.
 __device__ __forceinline__ int arow(const CountArgs &p, int v) { return p.rowmap ? p.rowmap[v] : v; }
-
-// Row start and length of v (int: m < 2^31 is enforced on the host).
-__device__ __forceinline__ void row_of(const int64_t *__restrict__ beg, int v, int &b, int &d) {
-  const long long lo = tc_ld_nc(beg + v), hi = tc_ld_nc(beg + v + 1);
-  b = (int)lo;
-  d = (int)(hi - lo);
-}
 
 // The list of class c.
 __device__ __forceinline__ const int *class_list(const CountArgs &p, int c) { return p.lists + p.off.off[c]; }
@@ -1083,7 +1009,7 @@ __global__ void __launch_bounds__(MAXT, MINB) count_kernel(CountArgs p) {
         const long long t_start = REC ? clock64() : 0;
         warp_vertex<SAME>(p, v, warp_tab, hits, wedges);
         if (REC && lane == 0) p.cycles[v] = (unsigned long long)(clock64() - t_start);
-        }
+      }
     }
   }
   drain_group_class<32, SAME, REC>(p, TC_CLASS_G32, warp_tab, hits, wedges);
@@ -1323,7 +1249,7 @@ __global__ void __launch_bounds__(512, 2) hub_kernel(CountArgs p, int log2C, int
         const int i = (bt << 5) + lane;
         int s = 0, dd = 0;
         if (i < dB) row_of(p.begC, tc_ld_nc(p.adjB + bB + i), s, dd);
-        if (p.split && dd > max(dA, p.table_min)) dd = 0;
+        if (p.split && dd > dA) dd = 0;
         probe_arcs<32, LongRow<32>::value>(p.adjC, s, dd, lane, tset, hits, wedges);
       }
     };

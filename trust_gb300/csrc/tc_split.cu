@@ -17,23 +17,9 @@
 #include "tc_count.h"
 #include "tc_internal.h"
 #include "tc_model.h"
+#include "tc_rows.cuh"
 
 namespace tc {
-
-// Position (0..31) of the n-th (0-based) set bit of mask; mask must have more than n set bits.
-__device__ __forceinline__ int split_nth_bit(unsigned mask, int n) {
-  int pos = 0;
-#pragma unroll
-  for (int step = 16; step >= 1; step >>= 1) {
-    const int cnt = __popc(mask & ((1u << step) - 1u));
-    if (n >= cnt) {
-      n -= cnt;
-      mask >>= step;
-      pos += step;
-    }
-  }
-  return pos;
-}
 
 // ---- traversal of the arcs ---------------------------------------------------------------------
 // Every arc (v,u) with d(v) >= 2 is visited once, in two phases.  Phase 1: a warp takes 32
@@ -85,7 +71,7 @@ __device__ __forceinline__ void short_arcs(const int64_t *__restrict__ beg, cons
     if (tot == 0) continue;
     const unsigned ne = __ballot_sync(TC_FULL_MASK, sd > 0);
     const int nc = __popc(ne);
-    const int src = lane < nc ? split_nth_bit(ne, lane) : 0;
+    const int src = lane < nc ? nth_set_bit(ne, lane) : 0;
     const int src_excl = __shfl_sync(TC_FULL_MASK, incl - sd, src);
     const int cexcl = lane < nc ? src_excl : 0x7fffffff;
     const int cbase = __shfl_sync(TC_FULL_MASK, b - (incl - sd), src);
@@ -616,7 +602,7 @@ __global__ void tile_sched_kernel(const int64_t *__restrict__ begA, const int64_
     if (tot == 0) continue;
     const unsigned ne = __ballot_sync(TC_FULL_MASK, sd > 0);
     const int nc = __popc(ne);
-    const int src = lane < nc ? split_nth_bit(ne, lane) : 0;
+    const int src = lane < nc ? nth_set_bit(ne, lane) : 0;
     const int src_excl = __shfl_sync(TC_FULL_MASK, incl - sd, src);
     const int cexcl = lane < nc ? src_excl : 0x7fffffff;
     const long long cbase = __shfl_sync(TC_FULL_MASK, b - (long long)(incl - sd), src);
