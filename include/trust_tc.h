@@ -108,16 +108,21 @@ typedef struct trust_tc_result {
                                a single-graph call, where it runs fused with classification) */
   double count_seconds;     /* CUDA-event time of the counting kernels alone (with the direction
                                split: from the first counting launch to the end of whichever of
-                               the two concurrent passes ends last)                          */
+                               the two concurrent kernels ends last, what is left of the rows'
+                               conversion to block bitmaps included; small graphs counted by one
+                               launch: the whole call)                                       */
   double call_seconds;      /* CUDA-event time of the whole device-side call                 */
   int64_t vertices;         /* n                                                            */
   int64_t edges;            /* m (oriented arcs = undirected edges)                         */
   int64_t max_out_degree;
-  int64_t wedges;           /* sum over arcs (v,u) with d(v)>=2 of d(u): the probe count     */
+  int64_t wedges;           /* sum over arcs (v,u) with d(v)>=2 of d(u), with the direction split
+                               of min(d(u), d(v)): the work in probes.  A measure, not the entries
+                               read: block bitmaps settle up to 16 of them with one lookup, and leave
+                               arcs between rows of at most 128 entries unsplit               */
   int64_t class_sizes[8];   /* vertices per schedule class (skip, g4, g8, g16, g32, warp, cta, cluster) */
   uint64_t *vertex_cycles;  /* caller-provided device array of n entries, or NULL            */
-  int32_t direction_split;  /* 1 when the second (reverse-direction) pass ran (tile loop: the
-                               number of jobs that ran it)                                  */
+  int32_t direction_split;  /* 1 when the arcs were split (tile loop: the number of jobs that
+                               were); 0 also where the split's scratch found no memory      */
   float split_saving_ms;    /* learned schedule: predicted saving of that pass, ms (else 0)  */
 } trust_tc_result;
 

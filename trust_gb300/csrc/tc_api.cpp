@@ -55,10 +55,11 @@ int ctx_init(trust_tc_ctx *c, int device) {
   TC_CUDA_TRY(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device));
   TC_CUDA_TRY(cudaDeviceGetAttribute(&c->max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   TC_CUDA_TRY(cudaDeviceGetAttribute(&c->clock_khz, cudaDevAttrClockRate, device));
-  static_assert(2 * sizeof(TcControl) % sizeof(int2) == 0, "alignment of the list behind");
-  TC_CUDA_TRY(cudaMalloc(&c->d_ctl, 2 * sizeof(TcControl) + sizeof(int2) * SMALL_MAX_UNITS));
-  c->d_small = c->d_ctl + 1;
-  c->d_small_units = reinterpret_cast<int2 *>(c->d_ctl + 2);
+  // the control block, the small path's accumulators and its list of pieces, each from a 256-byte boundary on
+  static_assert(sizeof(TcControl) <= 256, "one block each");
+  TC_CUDA_TRY(cudaMalloc(&c->d_ctl, 2 * 256 + sizeof(int2) * SMALL_MAX_UNITS));
+  c->d_small = reinterpret_cast<TcControl *>(reinterpret_cast<char *>(c->d_ctl) + 256);
+  c->d_small_units = reinterpret_cast<int2 *>(reinterpret_cast<char *>(c->d_ctl) + 512);
   TC_CUDA_TRY(cudaMallocHost(&c->h_ctl, sizeof(TcControl)));
   TC_CUDA_TRY(cudaMallocHost(&c->h_plans, TC_PLAN_WORDS * sizeof(unsigned long long)));
   for (auto &ev : c->ev) TC_CUDA_TRY(cudaEventCreate(&ev));
@@ -66,8 +67,8 @@ int ctx_init(trust_tc_ctx *c, int device) {
   for (auto &sl : c->staged) TC_CUDA_TRY(cudaEventCreateWithFlags(&sl.ready, cudaEventDisableTiming));
   TC_CUDA_TRY(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
   // zeroed here, not by the first call: the first call's stream may be capturing, and would only record it
+  // (the first call that uses them waits for it)
   TC_CUDA_TRY(cudaMemsetAsync(c->d_small, 0, sizeof(TcControl), c->copy_stream));
-  TC_CUDA_TRY(cudaStreamSynchronize(c->copy_stream));
   return TRUST_TC_OK;
 }
 
@@ -188,14 +189,16 @@ static int resolve_cfg(trust_tc_ctx *c, const trust_tc_opts &o, bool same, Launc
 // against 2335 ms, R-MAT 20 5.66 against 5.69 ms), so only outliers are promoted.
 constexpr float TC_PROMOTE_LOG2 = 26.f;
 
-// Below this many arcs the learned schedule's scheduling pass cannot be repaid: on R-MAT scale 18
-// (3.8M arcs, a 1.7 ms count) the split with the pass costs 2 % more than the tuned classes
-// without it, on scale 19 (7.7M arcs) it saves 5 %.  Smaller graphs run the tuned schedule.
+// Below this many arcs the learned schedule runs the tuned classes without its scheduling pass.  The line was
+// drawn where the pass and the split's two hash passes broke even (R-MAT 18, 3.8 M arcs: 2 % slower, R-MAT
+// 19, 7.7 M: 5 % faster).  With block bitmaps it lies lower, and this one has not been fitted again: forced split
+// / default, ms, R-MAT 17 0.60 / 0.71, R-MAT 18 0.92 / 1.65, R-MAT 18 with a = 0.45 1.13 / 0.79.
 constexpr int64_t TC_LEARNED_MIN_ARCS = (int64_t)1 << 22;
 // Nor where few arcs sit in long rows: the split pays through the probes of rows longer than
-// TC_LONG_ROW (128) entries.  Measured on GB300: it paid on every R-MAT graph with a >= 0.57
-// (scales 18-21; 34-67 % of arcs in such rows) and lost on a = 0.45 R-MAT and Chung-Lu graphs
-// (0-6 %), where the pass alone cost 0.3-1.0 ms more than the tuned classes.
+// TC_LONG_ROW (128) entries.  Measured on GB300 with the two hash passes: it paid on every R-MAT graph with
+// a >= 0.57 (scales 18-21; 34-67 % of arcs in such rows) and lost on a = 0.45 R-MAT and Chung-Lu graphs
+// (0-6 %), where the pass alone cost 0.3-1.0 ms more than the tuned classes.  With block bitmaps the same
+// side is right on all of these (Chung-Lu 3 M, 60 M edges, forced / default 11.1 / 8.5 ms).
 constexpr double TC_LEARNED_MIN_LONG_FRAC = 0.15;
 // Small graphs with long rows (fewer than 2^21 arcs, a row of at least 64 entries) run the plain
 // split, in 128-thread CTAs, under the learned schedule: packing 4 to 32 rows per warp leaves too few warp tasks to
@@ -324,7 +327,7 @@ static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust
     rc = small_count(c, g.begA, g.adjA, g.rows, g.mA, row_lo, row_hi < 0 ? g.rows : row_hi, check_ids, cfg.warp_max,
                      cfg.cta_max, st);
     if (rc) return rc;
-    const TcControl &h = *c->h_ctl;  // (read in place: a copy fetches more lines of what the GPU wrote, 0.8 us)
+    const TcControl &h = *c->h_ctl;  // (read in place, mostly its first 64 bytes: every further line of what the GPU wrote costs the host 0.5 us)
     if (h.status & TC_DEV_BAD_OFFSETS) return TRUST_TC_E_OFFSETS;
     if (h.status & TC_DEV_BAD_IDS) return TRUST_TC_E_IDS;
     float ms = 0;
@@ -412,8 +415,8 @@ static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust
       (o.direction_split == 1 || (learned && h.max_out_degree >= 64 && g.mA >= TC_LEARNED_MIN_ARCS &&
                                   (!fused || (double)h.long_arcs >= TC_LEARNED_MIN_LONG_FRAC * (double)g.mA)));
   // with the split (of one graph or of a tile job, below), rows longer than BITS_TABLE_MIN are counted as
-  // block bitmaps (tc_bits.cu) unless
-  // the caller asks for something of the hash tables' own: cycles, hub clusters, CTA bounds below
+  // block bitmaps (tc_bits.cu) unless the caller asks for something of the hash tables' own: cycles, hub
+  // clusters, CTA bounds below
   bool bits_ok = !o.record_cycles && o.hub_cluster == 0 && !o.test_wait_expiry &&
                        cfg.cta_max >= BITS_TABLE_MIN && bits_eligible(g, h.max_out_degree);
   unsigned long long plan_wedges = 0;
@@ -469,8 +472,8 @@ static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust
     } else if (o.direction_split == 1) {
       split = sorted;
     } else if (d_model) {
-      // predicted saving (warp-cycles spread over the resident warps) against the cost of the
-      // in-list build and second-pass setup, with a 1.5x margin
+      // predicted saving (warp-cycles spread over the resident warps) of the two hash passes against the
+      // cost of the in-list build and second-pass setup, with a 1.5x margin (the block bitmaps save more)
       const double warps = (double)c->num_sms * (double)std::max(cfg.blocks / std::max(c->num_sms, 1), 1) *
                            (double)(cfg.threads / 32);
       const double saved_ms = (double)plan.saved_cycles / (warps * (double)std::max(c->clock_khz, 1));
@@ -506,6 +509,7 @@ static int count_device_planned(trust_tc_ctx *c, const DevGraph3 &g, const trust
   }
   // a tile job (three CSRs, duplicate-free tables and probe rows): the same split, decided by the
   // probe totals of its plan
+  // (the arc gate is the one for whole graphs, not fitted to tile jobs)
   const bool consider3 = !same && g.split_ok && !g.rowmap && g.rows > 0 && g.min_deg == 1 &&
                          (o.direction_split == 1 ||
                           (o.direction_split < 0 && o.schedule == TRUST_TC_SCHED_LEARNED &&

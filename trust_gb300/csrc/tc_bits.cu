@@ -428,8 +428,8 @@ struct BitsArgs {
 // warp's four 8-lane groups drain, so that rows of any length keep the lanes busy.
 // Bound by the shared-memory and load pipe (R-MAT 22 a = 0.70: 71 % busy, 2.8 wavefronts per 16-bit
 // lookup of 32 lanes) and, on graphs whose rows exceed the L2 (R-MAT 22: 19 GB of DRAM reads in
-// 7.3 ms), by the latency of the row loads.  Counting time against the hash tables it replaces: R-MAT
-// 20 ef16 5.7 -> 1.0 ms, R-MAT 24 a = 0.70 163 -> 44 ms.
+// 7.3 ms), by the latency of the row loads.  The kernel takes 0.91 ms of R-MAT 20 ef16 and 32.4 of R-MAT 24
+// a = 0.70; the calls, against the two hash passes it replaces, 5.7 -> 2.4 ms and 170 -> 44.
 __device__ __forceinline__ u32 match4(const unsigned short *tab, uint4 e) {
   const unsigned char *t = reinterpret_cast<const unsigned char *>(tab);
   const u32 x0 = *reinterpret_cast<const unsigned short *>(t + (e.x >> 16)) & e.x;

@@ -56,8 +56,10 @@ struct trust_tc_ctx {
   size_t split_rowmap_cap = 0;
   int32_t *d_split_adj = nullptr;
   size_t split_adj_cap = 0;
-  int2 *d_small_units = nullptr;  // behind d_small: pieces of long rows
-  TcControl *d_small = nullptr;  // behind d_ctl: accumulators of the one-launch path, zero between calls
+  // behind d_ctl: the accumulators of the one-launch path, zero between calls, and its pieces of long rows
+  TcControl *d_small = nullptr;
+  int2 *d_small_units = nullptr;
+  bool small_zeroed = false;  // the accumulators' first zeroing has been waited for
   unsigned *d_bits_cols = nullptr;  // block-bitmap path: column popularity and ranks, counters, row lists
   size_t bits_cols_cap = 0;
   unsigned *d_bits_ent = nullptr;  // every row as block entries, then tail ids

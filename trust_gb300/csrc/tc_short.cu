@@ -7,7 +7,7 @@
 // are read coalesced, the rows' arcs fill the lanes without gaps, and each lane reads its arc's target
 // row (at most three 16-byte pieces) and compares it with its source row's keys, which the warp
 // staged in shared memory.
-// Bound by the load pipe (81 % busy: every lane reads its own two offsets and row) and its latency:
+// Bound by the load pipe (82 % busy: every lane reads its own two offsets and row) and its latency:
 // mesh 4096 x 4096 0.50 -> 0.36 ms of counting, the call 651 -> 490 us.  Rows to 8 beside longer
 // ones were tried too, with the target rows' pieces dealt over the lanes: Chung-Lu 3.8 M 433 -> 412
 // us but 160 -> 213 on 300,000 arcs and 120 us more on R-MAT 20, so mixed graphs keep the queues.

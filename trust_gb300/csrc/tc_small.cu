@@ -8,9 +8,9 @@
 // probes it, four rows at a time, eight lanes each; the last CTA to finish writes the totals
 // straight into the context's pinned control block and clears the accumulators.
 // Calls on GB300, general path / this one, us: R-MAT 8 (1,311 arcs) 79 / 27, R-MAT 16 ef16 (0.9 M)
-// 400 / 126, K_512 191 / 79, Erdos-Renyi 60,000 / 1.9 M arcs 161 / 133, one row of 15,000 entries 828
-// / 555.  Small graphs are bound by the launch and the round trip (device time 12 of R-MAT 8's 28 us),
-// R-MAT 16 by the issue of its 94 M probes.  Every other round of rows goes to the warps in reverse
+// 400 / 126, K_512 191 / 79, Erdos-Renyi 60,000 / 1.9 M arcs 161 / 133.
+// Small graphs are bound by the launch and the round trip (device time 12 of R-MAT 8's 28 us), R-MAT 16 by the
+// L1 (75 % busy) and the issue (68 %) of its 94 M probes.  Every other round of rows goes to the warps in reverse
 // order: with rows longest first a warp then gets about the same work (R-MAT 16 160 -> 142 us, R-MAT
 // 16 ef32 330 -> 244).  Tried and slower: chunks of 64 arcs whatever their rows (181 us).
 // Within a CTA the rows go to whichever warp is free, and a row too long for one warp (unoriented graphs, a
@@ -42,7 +42,8 @@ struct SmallArgs {
   int warp_max, cta_max;
   int splits;   // warps per row
   int words;    // bitmap words per warp; the last one stays zero (entries that are no ids)
-  TcControl *acc;    // device accumulators, zero between calls (bad_offset_at: CTAs finished, long_arcs: units)
+  TcControl *acc;    // device accumulators, zero between calls.  bad_offset_at: CTAs finished and, from bit 32
+                     // on, units: in the first line of what the host reads
   TcControl *out;    // pinned host block
   int2 *units;       // (row, first arc) of the long rows' pieces
 };
@@ -176,7 +177,7 @@ __device__ __forceinline__ void finish(const SmallArgs &p, SmallSums &cta, unsig
   }
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) cta.last = atomicAdd(&p.acc->bad_offset_at, 1ull) == gridDim.x - 1;
+  if (threadIdx.x == 0) cta.last = (unsigned)atomicAdd(&p.acc->bad_offset_at, 1ull) == gridDim.x - 1;
   __syncthreads();
   if (!cta.last) return;
   __threadfence();
@@ -248,7 +249,7 @@ __global__ void __launch_bounds__(SM_THREADS, 6) small_kernel(SmallArgs p) {
       if (part == 0) {
         const int per = unit_arcs(d), k = (d + per - 1) / per;
         unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(&p.acc->long_arcs, (unsigned long long)k);
+        if (lane == 0) at = atomicAdd(&p.acc->bad_offset_at, (unsigned long long)k << 32) >> 32;
         at = __shfl_sync(TC_FULL_MASK, at, 0);
         if (at + k > SMALL_MAX_UNITS) bad |= TC_DEV_BAD_OFFSETS;  // rows that overlap
         else
@@ -316,6 +317,10 @@ bool small_graph(int64_t n, int64_t m) { return n >= 1 && n <= SMALL_MAX_IDS && 
 
 int small_count(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t n, int64_t m, int64_t row_lo,
                 int64_t row_hi, int check_ids, int warp_max, int cta_max, cudaStream_t st) {
+  if (!c->small_zeroed) {
+    TC_CUDA_TRY(cudaStreamSynchronize(c->copy_stream));
+    c->small_zeroed = true;
+  }
   SmallArgs a;
   a.beg = beg;
   a.adj = adj;
@@ -343,7 +348,7 @@ int small_count(trust_tc_ctx *c, const int64_t *beg, const int32_t *adj, int64_t
   TC_CUDA_TRY(cudaGetLastError());
   TC_CUDA_TRY(cudaEventRecord(c->ev[4], st));
   TC_CUDA_TRY(cudaStreamSynchronize(st));
-  const int n_units = (int)c->h_ctl->long_arcs;
+  const int n_units = (int)(c->h_ctl->bad_offset_at >> 32);
   if (n_units == 0 || c->h_ctl->status) return TRUST_TC_OK;
   const TcControl rest = *c->h_ctl;
   long_rows_kernel<<<std::min(n_units, c->num_sms * 6), SM_THREADS, sizeof(unsigned) * (size_t)a.words, st>>>(a, n_units);
