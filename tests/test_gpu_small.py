@@ -154,27 +154,53 @@ def test_overlapping_rows_end_early(ctx, length):
     assert T.count_csr(*_dev(*O.build_csr(ok, 40)), ctx=ctx).triangles == tri
 
 
+_CAPTURE = """
+import ctypes as C
+import torch
+import trust_gb300 as T
+from trust_gb300 import _lib
+from oracle import oracle as O
+from tests import graphs
+pairs, expect = graphs.complete(60)
+db, da = (torch.from_numpy(x).cuda() for x in O.build_csr(pairs, 60))
+# no zeroed memory by chance: freed blocks of the accumulators' size that held offsets
+dirty, lib, p = [], T.load(), torch.from_numpy(pairs).cuda()
+for _ in range(64):
+    x = [C.c_void_p(), C.c_void_p(), C.c_int64(), C.c_int64()]
+    T.check(lib.trust_tc_build_csr_device(None, C.c_void_p(p.data_ptr()), p.shape[0], 60, *[C.byref(y) for y in x]), "")
+    dirty.append(x)
+for x in dirty:
+    lib.trust_tc_free_device(x[0])
+with T.Context() as c:
+    s = torch.cuda.Stream()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(s):
+        g.capture_begin(capture_error_mode="relaxed")
+        try:
+            T.count_csr(db, da, ctx=c, stream=s.cuda_stream)
+            status = _lib.OK
+        except T.TrustTcError as e:
+            status = e.status
+        try:
+            g.capture_end()
+        except RuntimeError:  # the capture is invalid
+            pass
+    assert status == _lib.E_CUDA, status
+    for _ in range(2):
+        assert T.count_csr(db, da, ctx=c).triangles == expect
+print("counted")
+"""
+
+
 def test_first_call_on_a_capturing_stream():
-    """A call cannot be captured (it synchronises): it fails, and the context's next call counts."""
-    beg, adj = O.build_csr(graphs.complete(60)[0], 60)
-    db, da = _dev(beg, adj)
-    dirty = [torch.full((64,), -1, dtype=torch.int64, device="cuda") for _ in range(64)]  # no zeroed memory by chance
-    del dirty
-    torch.cuda.empty_cache()
-    with T.Context() as c:
-        s = torch.cuda.Stream()
-        g = torch.cuda.CUDAGraph()
-        with torch.cuda.stream(s):
-            g.capture_begin(capture_error_mode="relaxed")
-            with pytest.raises(T.TrustTcError) as e:
-                T.count_csr(db, da, ctx=c, stream=s.cuda_stream)
-            try:
-                g.capture_end()
-            except RuntimeError:  # the capture is invalid
-                pass
-        assert e.value.status == _lib.E_CUDA
-        for _ in range(2):
-            assert T.count_csr(db, da, ctx=c).triangles == graphs.complete(60)[1]
+    """A call cannot be captured (it synchronises): it fails, and the context's next call counts.  In a
+    process of its own: torch's allocator keeps a failed capture's state."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _CAPTURE], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "counted", r.stderr[-2000:]
 
 
 def test_callers_streams_and_contexts_at_once():
